@@ -62,10 +62,10 @@ __device__ __forceinline__ void blend_probe_fp32(const DeviceGrid& g, uint32_t p
             for (uint32_t r = 0; r < R; ++r) {
                 float4 d = s_dirs[r];
                 float4 v = s_rays[r];
-                float w = fmaxf(0.0f, td.x * d.x + td.y * d.y + td.z * d.z);
-                a0 += w * v.x;
-                a1 += w * v.y;
-                a2 += w * v.z;
+                float w = blend_cosine(td, d);
+                a0 = blend_add(w, v.x, a0);
+                a1 = blend_add(w, v.y, a1);
+                a2 = blend_add(w, v.z, a2);
                 aw += w;
             }
             if (aw > 1e-3f) {
@@ -78,8 +78,8 @@ __device__ __forceinline__ void blend_probe_fp32(const DeviceGrid& g, uint32_t p
             float4 prev = *texel;
             float mc = fmaxf(fmaxf(fabsf(a0 - prev.x), fabsf(a1 - prev.y)), fabsf(a2 - prev.z));
             atomicMax(&s_max_change, __float_as_uint(mc));
-            *texel = store_color(g, a0 * (1.0f - hy) + prev.x * hy, a1 * (1.0f - hy) + prev.y * hy,
-                                 a2 * (1.0f - hy) + prev.z * hy);
+            *texel = store_color(g, blend_hysteresis(a0, prev.x, hy), blend_hysteresis(a1, prev.y, hy),
+                                 blend_hysteresis(a2, prev.z, hy));
         } else {
             int u = t - ncol;
             int tx = u % nd, ty = u / nd;
@@ -91,9 +91,9 @@ __device__ __forceinline__ void blend_probe_fp32(const DeviceGrid& g, uint32_t p
                 float4 d = s_dirs[r];
                 float dep = fminf(cl, s_rays[r].w);
                 if (dep < 0.0f) dep = cl;
-                float w = powf(fmaxf(0.0f, td.x * d.x + td.y * d.y + td.z * d.z), g.sharp);
-                a0 += w * dep;
-                a1 += w * dep * dep;
+                float w = powf(blend_cosine(td, d), g.sharp);
+                a0 = blend_add(w, dep, a0);
+                a1 = blend_add_square(w, dep, a1);
                 aw += w;
             }
             if (aw > 1e-3f) {
@@ -103,7 +103,7 @@ __device__ __forceinline__ void blend_probe_fp32(const DeviceGrid& g, uint32_t p
             size_t px = (size_t)((int)g.depth_res * tile + 1 + tx), py = (size_t)((int)g.depth_res * iz + 1 + ty);
             float2* texel = depth + py * g.depth_w + px;
             float2 prev = *texel;
-            *texel = store_depth(g, a0 * (1.0f - hy) + prev.x * hy, a1 * (1.0f - hy) + prev.y * hy);
+            *texel = store_depth(g, blend_hysteresis(a0, prev.x, hy), blend_hysteresis(a1, prev.y, hy));
         }
     }
     __syncthreads();

@@ -149,6 +149,20 @@ __device__ __forceinline__ float2 store_depth(const DeviceGrid& g, float m, floa
     return make_float2(m, m2);
 }
 
+// The FP32 blend's arithmetic, with its multiply-adds written out so that the
+// per-probe kernel and the shared-weight kernel give the same bits whatever
+// the code around them looks like: cosine weight of ray direction d in texel
+// direction t, one ray's share of a sum, of the depth moments, and the
+// hysteresis step.
+__device__ __forceinline__ float blend_cosine(float3 t, float4 d) {
+    return fmaxf(0.0f, fmaf(t.z, d.z, fmaf(t.x, d.x, __fmul_rn(t.y, d.y))));
+}
+__device__ __forceinline__ float blend_add(float w, float v, float sum) { return fmaf(w, v, sum); }
+__device__ __forceinline__ float blend_add_square(float w, float v, float sum) { return fmaf(__fmul_rn(w, v), v, sum); }
+__device__ __forceinline__ float blend_hysteresis(float now, float prev, float hy) {
+    return fmaf(now, 1.0f - hy, __fmul_rn(prev, hy));
+}
+
 struct DeviceLight {
     float dir[3], color[3], sky[3];
     float sun_brightness;  // LightBuffer.color.a: the atmospheric sky's sun factor

@@ -2258,7 +2258,8 @@ ddgi_status ddgi_backward(ddgi_ctx* ctx, const float* dL_dcolor, size_t bytes, f
             ddgi_status s = upload_dirs(ctx, &ctx->rec_orient[9 * (size_t)v], st);
             if (s != DDGI_OK) return s;
             CK(launch_replay_update(sc, ctx->dg, ctx->dl, ctx->dirs, ctx->work_states, ctx->work_color, ctx->work_depth,
-                                    ctx->rec_thit + rays * v, ctx->rec_prim + rays * v, ctx->rays, ctx->err, st),
+                                    ctx->rec_thit + rays * v, ctx->rec_prim + rays * v, ctx->rays,
+                                    reinterpret_cast<float*>(ctx->tc_weights), ctx->tc_rowsum, ctx->err, st),
                "replay");
         }
         CK(cudaMemcpyAsync(ctx->work_states, ctx->rec_states, sizeof(uint32_t) * P, cudaMemcpyDeviceToDevice, st),

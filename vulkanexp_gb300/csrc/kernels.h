@@ -22,6 +22,15 @@ inline cudaError_t ensure_dynamic_smem(K* kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+// Multiprocessors of the current device.
+inline uint32_t sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        return 1u;
+    return (uint32_t)sms;
+}
+
 // trace.cu
 cudaError_t launch_trace_shade(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L,
                                const uint32_t* probe_list, uint32_t nprobes, const float4* dirs,
@@ -185,7 +194,8 @@ cudaError_t launch_final_gather(const GatherArgs& a, const void* color, const vo
 // adjoint.cu
 cudaError_t launch_replay_update(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L, const float4* dirs,
                                  uint32_t* states, float4* color, float2* depth, const float4* thit,
-                                 const uint32_t* prim, float4* rays, uint32_t* err, cudaStream_t st);
+                                 const uint32_t* prim, float4* rays, float* W, float* wsum, uint32_t* err,
+                                 cudaStream_t st);
 cudaError_t launch_adjoint_step(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L, const float4* dirs,
                                 const uint32_t* states, const float4* color_prev, const float2* depth_prev,
                                 const float4* thit, const uint32_t* prim, float4* gk, float4* gprev, float4* gx,
