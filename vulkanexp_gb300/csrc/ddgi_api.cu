@@ -111,6 +111,7 @@ DeviceGrid make_device_grid(const ddgi_grid_desc& g) {
         d.res[k] = g.resolution[k];
         volatile float diff = g.extent_max[k] - g.extent_min[k];
         d.cell[k] = diff / (float)(g.resolution[k] - 1);
+        d.inv_cell[k] = 1.0f / d.cell[k];
     }
     {
         volatile float a = d.cell[0] * d.cell[0];

@@ -230,10 +230,11 @@ __global__ void __launch_bounds__(128) k_shade_classify(DeviceGrid g, DeviceLigh
 // Shading, pass 2, one thread per queued front hit: closesthit.glsl
 // (NO_REFLECTION) up to the shadow query, whose rays are appended to the
 // shadow queue (an unshadowed ray later adds the sun term).
-// Built for eight resident blocks per SM (64 registers): 0.05 ms faster per
-// update than six (80 registers, no spill) on the 1M-triangle terrain.
+// Built for five resident blocks per SM (96 registers): 366 us for the hits of
+// the 1M-triangle terrain update against 373 us at six and 396 us at four; 23,
+// 25 and 22 us for the 65 K hits of a small room.
 template <class AV>
-__global__ void __launch_bounds__(128, 8) k_shade_front(DeviceScene sc, DeviceGrid g, DeviceLight L,
+__global__ void __launch_bounds__(128, 5) k_shade_front(DeviceScene sc, DeviceGrid g, DeviceLight L,
                                                         const uint32_t* __restrict__ probe_list,
                                                         const float4* __restrict__ dirs,
                                                         const uint32_t* __restrict__ states, AV at, WaveHits hits,
@@ -436,9 +437,10 @@ __global__ void __launch_bounds__(128) k_batch_classify(BatchTables bt, uint32_t
 
 // Batched shading, pass 2 (k_shade_front with the volume's scene, grid,
 // light, states and atlas; the shadow-queue entry carries the volume).
-// Eight resident blocks per SM, like k_shade_front: the 48-volume batch
-// update 30.4 -> 29.9 ms against six.
-__global__ void __launch_bounds__(128, 8) k_batch_shade_front(BatchTables bt, WaveHits hits,
+// Four resident blocks per SM (the volume's tables take registers that the
+// other form has in constants): a twelve-volume update 5.88 ms against 5.95 ms
+// at five and 6.00 ms at six.
+__global__ void __launch_bounds__(128, 4) k_batch_shade_front(BatchTables bt, WaveHits hits,
                                                               const uint32_t* front_count, float4* rays_out,
                                                               ShadowQueue q) {
     const uint32_t n = *front_count;
