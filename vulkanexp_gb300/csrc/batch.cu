@@ -56,7 +56,7 @@ struct ddgi_batch {
     std::vector<uint64_t> scene_builds;
     std::vector<ddgi_grid_desc> grids;
     // arena
-    BvhNode* nodes = nullptr;
+    WalkNode* walk = nullptr;  // nodes
     BvhTri* tris = nullptr;
     GpuInstance* insts = nullptr;
     uint64_t node_count = 0, tri_count = 0, inst_count = 0;
@@ -153,24 +153,21 @@ constexpr uint32_t kGroups = 4;  // volume groups of the graph's branches
 // Node references of a volume's trees moved into the arena: inner nodes by
 // node_off; leaves of the mesh trees (node index < tlas_start) by tri_off,
 // leaves of the top-level tree by inst_off.
-__global__ void k_rebase_nodes(const BvhNode* __restrict__ src, uint32_t n, uint32_t tlas_start, int node_off,
-                               int tri_off, int inst_off, BvhNode* __restrict__ dst) {
+__global__ void k_rebase_nodes(const WalkNode* __restrict__ src, uint32_t n, uint32_t tlas_start, int node_off,
+                               int tri_off, int inst_off, WalkNode* __restrict__ dst) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    BvhNode nd = src[i];
+    WalkNode nd = src[i];
     const int prim_off = i >= tlas_start ? inst_off : tri_off;
-    int r[2] = {nd.d.x, nd.d.y};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        if (r[k] >= 0) {
-            r[k] += node_off;
+        if (nd.ref[k] >= 0) {
+            nd.ref[k] += node_off;
         } else {
-            int first = (~r[k]) >> 3, cnt = (~r[k]) & 7;
-            r[k] = ~(((first + prim_off) << 3) | cnt);
+            int first = (~nd.ref[k]) >> 3, cnt = (~nd.ref[k]) & 7;
+            nd.ref[k] = ~(((first + prim_off) << 3) | cnt);
         }
     }
-    nd.d.x = r[0];
-    nd.d.y = r[1];
     dst[i] = nd;
 }
 
@@ -239,7 +236,7 @@ BatchTables tables(const ddgi_batch* b) {
 
 DeviceScene arena_scene(const ddgi_batch* b) {
     DeviceScene s{};
-    s.nodes = b->nodes;
+    s.walk = b->walk;
     s.tris = b->tris;
     s.instances = b->insts;
     s.tlas_root = -1;
@@ -538,7 +535,7 @@ ddgi_status ddgi_batch_create(ddgi_ctx* const* volumes, uint32_t count, ddgi_str
 
     // ---- allocations ----
     const size_t N = std::max<uint64_t>(rays, 1);
-    if (cudaMalloc(&b->nodes, sizeof(BvhNode) * std::max<uint64_t>(nodes, 1)) != cudaSuccess ||
+    if (cudaMalloc(&b->walk, sizeof(WalkNode) * std::max<uint64_t>(nodes, 1)) != cudaSuccess ||
         cudaMalloc(&b->tris, sizeof(BvhTri) * std::max<uint64_t>(tris, 1)) != cudaSuccess ||
         cudaMalloc(&b->insts, sizeof(GpuInstance) * std::max<uint64_t>(insts, 1)) != cudaSuccess ||
         cudaMalloc(&b->wnodes, sizeof(WideNode) * std::max<uint64_t>(b->wnode_count, 1)) != cudaSuccess ||
@@ -661,8 +658,8 @@ ddgi_status ddgi_batch_create(ddgi_ctx* const* volumes, uint32_t count, ddgi_str
         const uint32_t n = (uint32_t)S.node_count;
         if (n > 0) {
             const uint32_t tlas_start = S.tlas_root >= 0 ? (uint32_t)S.tlas_root : n;
-            k_rebase_nodes<<<(n + 255) / 256, 256, 0, st>>>(S.nodes, n, tlas_start, (int)node_off, (int)tri_off,
-                                                            (int)inst_off, b->nodes + node_off);
+            k_rebase_nodes<<<(n + 255) / 256, 256, 0, st>>>(S.walk, n, tlas_start, (int)node_off, (int)tri_off,
+                                                            (int)inst_off, b->walk + node_off);
         }
         if (S.tri_count > 0 &&
             cudaMemcpyAsync(b->tris + tri_off, S.tris, sizeof(BvhTri) * S.tri_count, cudaMemcpyDeviceToDevice, st) !=
@@ -697,7 +694,7 @@ ddgi_status ddgi_batch_destroy(ddgi_batch* b) {
     if (!b) return DDGI_OK;
     if (b->pending) wait_event(b, b->done_ev, 60000);
     drop_graph(b);
-    bfree(b->nodes);
+    bfree(b->walk);
     bfree(b->tris);
     bfree(b->insts);
     bfree(b->wnodes);

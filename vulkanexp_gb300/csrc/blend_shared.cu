@@ -36,27 +36,6 @@ constexpr uint32_t kWeightTexels = 8;
 constexpr uint32_t kBlendThreads = 288;
 constexpr uint32_t kBatchTile = 4;  // probes per work item of a batch
 
-// Two floats in one 64-bit register: Blackwell's packed FP32 instructions
-// round each half as the scalar ones do.
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float* a, float* b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // Weights of kWeightTexels texels from `t0` over all rays, by one block: a
 // thread computes every 32nd ray's weight of one texel (the powers of the
 // depth weights are the cost), then eight threads add up the texels' sums in

@@ -58,6 +58,22 @@ struct __align__(16) BvhNode {
 };
 static_assert(sizeof(BvhNode) == 64, "node is 64 bytes");
 
+// The same node as the persistent walkers read it, 64 bytes in two 256-bit
+// loads: per child the box as centre and half extent (rounded so that it
+// holds the node's box), the coordinates paired for the packed FP32
+// instructions, and the references between them:
+//   c0.x c0.y | c1.x c1.y | c0.z c1.z | ref0 ref1
+//   h0.x h0.y | h1.x h1.y | h0.z h1.z | unused
+// A box that is never hit has half extents of -infinity, one that overflowed
+// +infinity about zero.
+struct __align__(32) WalkNode {
+    float c0[2], c1[2], cz[2];
+    int32_t ref[2];
+    float h0[2], h1[2], hz[2];
+    uint32_t unused[2];
+};
+static_assert(sizeof(WalkNode) == 64, "walk node is 64 bytes");
+
 // Triangle in leaf order, 48 bytes: v0 (w = primitive id), v1, v2.
 struct __align__(16) BvhTri {
     float4 v0, v1, v2;
@@ -99,6 +115,7 @@ constexpr uint32_t kMaxWideNodes = 0x7FFFFFu;
 
 struct DeviceScene {
     const BvhNode* nodes;
+    const WalkNode* walk;  // the nodes in the persistent walkers' form
     const BvhTri* tris;
     const GpuInstance* instances;        // leaf order (traversal)
     const GpuInstance* instances_by_id;  // caller order (shading)
@@ -248,6 +265,32 @@ __device__ __forceinline__ void xform_exact(const float4 w[3], float3 o, float3 
     }
     *oo = make_float3(r[0], r[1], r[2]);
     *od = make_float3(s[0], s[1], s[2]);
+}
+
+// Two floats in one 64-bit register: Blackwell's packed FP32 instructions
+// round each half as the scalar ones do.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float* a, float* b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // Three-input min / max (PTX min.f32 / max.f32 with three sources, sm_100

@@ -29,6 +29,7 @@ constexpr int kMaxStack = 96;
 
 struct SceneBuffers {
     BvhNode* nodes = nullptr;
+    WalkNode* walk = nullptr;  // the nodes as the persistent walkers read them
     BvhTri* tris = nullptr;
     GpuInstance* inst_leaf = nullptr;
     GpuInstance* inst_id = nullptr;
@@ -204,6 +205,7 @@ inline std::vector<uint32_t> probe_morton_order(const int32_t res[3]) {
 inline DeviceScene device_scene(const ddgi_ctx* c) {
     DeviceScene s{};
     s.nodes = c->scene.nodes;
+    s.walk = c->scene.walk;
     s.tris = c->scene.tris;
     s.instances = c->scene.inst_leaf;
     s.instances_by_id = c->scene.inst_id;

@@ -165,6 +165,7 @@ void free_scene(SceneBuffers& s) {
     dfree(s.sub_lo);
     dfree(s.sub_hi);
     dfree(s.nodes);
+    dfree(s.walk);
     dfree(s.tris);
     dfree(s.inst_leaf);
     dfree(s.inst_id);
@@ -1040,6 +1041,7 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
         return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "scene too large (%llu triangles)", (unsigned long long)total_tris);
     }
     CKB(cudaMalloc(&S.nodes, sizeof(BvhNode) * std::max<uint64_t>(total_nodes + tlas_nodes, 1)), "alloc nodes");
+    CKB(cudaMalloc(&S.walk, sizeof(WalkNode) * std::max<uint64_t>(total_nodes + tlas_nodes, 1)), "alloc nodes");
     CKB(cudaMalloc(&S.tris, sizeof(BvhTri) * std::max<uint64_t>(total_tris, 1)), "alloc triangles");
     CKB(cudaMalloc(&S.inst_leaf, sizeof(GpuInstance) * std::max<uint32_t>(ni, 1)), "alloc instances");
     CKB(cudaMalloc(&S.inst_id, sizeof(GpuInstance) * std::max<uint32_t>(ni, 1)), "alloc instances");
@@ -1186,6 +1188,14 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
             return ls;
         }
     }
+    {
+        cudaError_t e = launch_walk_nodes(S.nodes, (uint32_t)S.node_count, S.walk, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the build is complete on return
+        if (e != cudaSuccess) {
+            free_scene(ctx->scene);
+            return cuda_fail(ctx, e, "walk nodes");
+        }
+    }
     S.build_id = next_build_id();
     S.built = true;
     if (ctx->tune.node_width == 8) {  // the wide copies are made when first asked for
@@ -1292,6 +1302,7 @@ ddgi_status ddgi_update_instances(ddgi_ctx* ctx, const uint32_t* ids, const floa
            "top-level refit");
         // the host vectors above are staged by the copies before they return
     }
+    CK(launch_walk_nodes(S.nodes + S.tlas_root, ni > 1 ? ni - 1 : 1, S.walk + S.tlas_root, st), "walk nodes");
     {
         ddgi_status ws = refresh_wide_top(ctx, st);
         if (ws != DDGI_OK) return ws;

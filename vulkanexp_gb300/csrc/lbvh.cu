@@ -553,4 +553,50 @@ cudaError_t gather_mesh_tris(const float4* pos, const uint32_t* indices, uint32_
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Nodes in the walkers' form
+// ---------------------------------------------------------------------------
+namespace {
+
+// One child's interval along one axis as centre and half extent: the half
+// extent is rounded up from the farther plane, so the interval holds [lo, hi].
+__device__ __forceinline__ void centre_half(float lo, float hi, float* c, float* h) {
+    if (!(lo <= hi)) {  // never hit
+        *c = 0.0f;
+        *h = -INFINITY;
+        return;
+    }
+    *c = 0.5f * lo + 0.5f * hi;
+    *h = fmaxf(__fsub_ru(hi, *c), __fsub_ru(*c, lo));
+    if (!isfinite(*c) || !isfinite(*h)) {  // a plane overflowed: always hit
+        *c = 0.0f;
+        *h = INFINITY;
+    }
+}
+
+__global__ void k_walk_nodes(const BvhNode* __restrict__ nodes, uint32_t n, WalkNode* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const BvhNode b = nodes[i];
+    WalkNode w;
+    centre_half(b.a.x, b.a.y, &w.c0[0], &w.h0[0]);
+    centre_half(b.a.z, b.a.w, &w.c0[1], &w.h0[1]);
+    centre_half(b.b.x, b.b.y, &w.c1[0], &w.h1[0]);
+    centre_half(b.b.z, b.b.w, &w.c1[1], &w.h1[1]);
+    centre_half(b.c.x, b.c.y, &w.cz[0], &w.hz[0]);
+    centre_half(b.c.z, b.c.w, &w.cz[1], &w.hz[1]);
+    w.ref[0] = b.d.x;
+    w.ref[1] = b.d.y;
+    w.unused[0] = w.unused[1] = 0u;
+    out[i] = w;
+}
+
+}  // namespace
+
+cudaError_t launch_walk_nodes(const BvhNode* nodes, uint32_t n, WalkNode* out, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    k_walk_nodes<<<(n + 255) / 256, 256, 0, st>>>(nodes, n, out);
+    return cudaGetLastError();
+}
+
 }  // namespace ddgi

@@ -42,4 +42,7 @@ cudaError_t lbvh_refit_top(BvhNode* nodes, int node_base, const float4* leaf_lo,
                            const uint32_t* leaf_parent, const uint32_t* node_parent, uint32_t* flags, float4* sub_lo,
                            float4* sub_hi, uint32_t* err, cudaStream_t st);
 
+// The `n` nodes from `nodes` in the persistent walkers' form.
+cudaError_t launch_walk_nodes(const BvhNode* nodes, uint32_t n, WalkNode* out, cudaStream_t st);
+
 }  // namespace ddgi

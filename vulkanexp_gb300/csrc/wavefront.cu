@@ -44,6 +44,8 @@ __device__ __forceinline__ void grouped_ray(uint32_t id, uint32_t R, uint32_t rp
 }
 
 struct PrimaryJob {
+    static constexpr float kTmin = 0.01f;
+    static constexpr uint32_t kMask = 0x3u;
     DeviceGrid g;
     const uint32_t* probe_list;
     const float4* dirs;
@@ -68,7 +70,7 @@ struct PrimaryJob {
         uint32_t probe = probe_list ? __ldg(probe_list + slot) : slot;
         *out = slot * R + ray;
         float4 d4 = __ldg(dirs + ray);
-        return w.start(sc, probe_origin_exact(g, probe), f3(d4.x, d4.y, d4.z), 0.01f, g.tmax, 0x3u);
+        return w.start(sc, probe_origin_exact(g, probe), f3(d4.x, d4.y, d4.z), g.tmax);
     }
     template <class W>
     __device__ __forceinline__ void finish(const W& w, uint32_t out) const {
@@ -79,6 +81,8 @@ struct PrimaryJob {
 };
 
 struct ShadowJob {
+    static constexpr float kTmin = 0.1f;
+    static constexpr uint32_t kMask = 0xFFu;
     const ShadowQueue q;
     float3 dir;
     float4* rays;
@@ -89,7 +93,7 @@ struct ShadowJob {
     __device__ __forceinline__ bool start(W& w, const DeviceScene& sc, uint32_t id, uint32_t* out) const {
         *out = id;
         float4 p = q.pos[id];
-        return w.start(sc, f3(p.x, p.y, p.z), dir, 0.1f, 10000.0f, 0xFFu);
+        return w.start(sc, f3(p.x, p.y, p.z), dir, 10000.0f);
     }
     template <class W>
     __device__ __forceinline__ void finish(const W& w, uint32_t id) const {
@@ -138,10 +142,12 @@ __device__ __forceinline__ void persistent_walk(const DeviceScene& sc, const Job
     w.cap = stack_cap;
     w.clear();
     w.wait_max = knobs.wait;
+    w.tmin = Job::kTmin;
+    w.mask = Job::kMask;
     bool active = false;
     bool drained = false;  // warp-uniform: the work counter has passed `total`
     uint32_t out = 0;
-    for (;;) {
+    for (uint32_t calls = 0;; ++calls) {
         unsigned busy = __ballot_sync(kFull, active);
         const unsigned idle = ~busy;
         if (!drained && (__popc(idle) >= refill || busy == 0)) {
@@ -163,7 +169,7 @@ __device__ __forceinline__ void persistent_walk(const DeviceScene& sc, const Job
             if (drained) break;
             continue;
         }
-        bool fin = w.advance(sc, err, active);  // every lane takes part (warp votes)
+        bool fin = w.advance(sc, err, active, calls);  // every lane takes part (warp votes)
         if (active && fin) {
             job.finish(w, out);
             active = false;
@@ -276,6 +282,8 @@ __global__ void __launch_bounds__(128, 5) k_shade_front(DeviceScene sc, DeviceGr
 // on every axis (hit position rounded product, then sum).
 // ---------------------------------------------------------------------------
 struct InitJob {
+    static constexpr float kTmin = 0.01f;
+    static constexpr uint32_t kMask = 0x1u;
     DeviceGrid g;
     const float4* dirs;  // kInitRays directions
     float tmax;
@@ -287,7 +295,7 @@ struct InitJob {
         *out = id;
         const uint32_t probe = id / kInitRays, i = id - probe * kInitRays;
         float4 d4 = __ldg(dirs + i);
-        return w.start(sc, probe_origin_exact(g, probe), f3(d4.x, d4.y, d4.z), 0.01f, tmax, 0x1u);
+        return w.start(sc, probe_origin_exact(g, probe), f3(d4.x, d4.y, d4.z), tmax);
     }
     template <class W>
     __device__ __forceinline__ void finish(const W& w, uint32_t id) const {
@@ -332,6 +340,8 @@ __device__ __forceinline__ uint32_t batch_volume(const BatchTables& bt, uint32_t
 }
 
 struct BatchPrimaryJob {
+    static constexpr float kTmin = 0.01f;
+    static constexpr uint32_t kMask = 0x3u;
     BatchTables bt;
     WaveHits hits;
 
@@ -355,7 +365,7 @@ struct BatchPrimaryJob {
         *out = base + slot * R + ray;
         float4 d4 = __ldg(bt.dirs + vol.dir_base + ray);
         return w.start_at(sc, W::kWide ? vol.wroot : vol.root, probe_origin_exact(vol.g, slot), f3(d4.x, d4.y, d4.z),
-                          0.01f, vol.g.tmax, 0x3u);
+                          vol.g.tmax);
     }
     template <class W>
     __device__ __forceinline__ void finish(const W& w, uint32_t out) const {
@@ -366,6 +376,8 @@ struct BatchPrimaryJob {
 };
 
 struct BatchShadowJob {
+    static constexpr float kTmin = 0.1f;
+    static constexpr uint32_t kMask = 0xFFu;
     const ShadowQueue q;
     BatchTables bt;
     float4* rays;
@@ -382,7 +394,7 @@ struct BatchShadowJob {
         }
         const BatchVolume& vol = bt.vols[v];
         return w.start_at(sc, W::kWide ? vol.wroot : vol.root, f3(p.x, p.y, p.z),
-                          f3(vol.L.dir[0], vol.L.dir[1], vol.L.dir[2]), 0.1f, 10000.0f, 0xFFu);
+                          f3(vol.L.dir[0], vol.L.dir[1], vol.L.dir[2]), 10000.0f);
     }
     template <class W>
     __device__ __forceinline__ void finish(const W& w, uint32_t id) const {
@@ -474,6 +486,9 @@ __global__ void __launch_bounds__(128, 4) k_batch_shade_front(BatchTables bt, Wa
     }
 }
 
+// Shared memory of a block's stacks.
+size_t walker_smem(int entries) { return (size_t)entries * kPersistThreads * sizeof(int); }
+
 uint32_t persistent_blocks(const void* kernel, size_t smem, uint32_t cap_per_sm = 0) {
     static int sms = 0;
     if (sms == 0) {
@@ -500,7 +515,7 @@ cudaError_t wavefront_kernels(const DeviceScene& sc, const DeviceGrid& g, const 
                               uint32_t* counters, float4* rays_out, ddgi_hit* hits_out, int stack_cap, int split,
                               uint32_t* err, cudaStream_t st, cudaEvent_t after_primary, const uint32_t* dev_count,
                               const TraceTuning& tune, const PrimaryJob& pj) {
-    const size_t smem = (size_t)split * kPersistThreads * sizeof(int);
+    const size_t smem = walker_smem(split);
     const WalkKnobs knobs = walk_knobs(tune);
     k_primary<Stack, Walker><<<persistent_blocks((const void*)k_primary<Stack, Walker>, smem, tune.ctas_per_sm),
                                kPersistThreads, smem, st>>>(sc, pj, counters, stack_cap, split, knobs, err);
@@ -569,7 +584,7 @@ cudaError_t batch_trace_kernels(const DeviceScene& arena, const BatchTables& bt,
                                 ShadowQueue q, uint32_t* counters, float4* rays_out, int stack_cap, int split,
                                 const TraceTuning& tune, cudaStream_t st, cudaEvent_t after_primary,
                                 cudaEvent_t after_shade) {
-    const size_t smem = (size_t)split * kPersistThreads * sizeof(int);
+    const size_t smem = walker_smem(split);
     const WalkKnobs knobs = walk_knobs(tune);
     BatchPrimaryJob pj{bt, hits};
     k_batch_primary<Stack, Walker>
@@ -623,7 +638,7 @@ cudaError_t launch_init_probes(const DeviceScene& sc, const DeviceGrid& g, const
     if (e == cudaSuccess) e = cudaMemsetAsync(near, 0, sizeof(uint32_t) * P, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    const size_t smem = (size_t)stack_cap * kPersistThreads * sizeof(int);
+    const size_t smem = walker_smem(stack_cap);
     InitJob job{g, dirs, 1.5f * g.cell_len, back, near};
     k_init_probes<<<persistent_blocks((const void*)k_init_probes, smem), kPersistThreads, smem, st>>>(
         sc, job, P * kInitRays, counters, stack_cap, err);
