@@ -13,8 +13,8 @@
 // sun or sky once the hits are fixed, so only the colour chain is reversed.
 //
 // Reverse step k, given G_k = dL/d atlas_k:
-//   k_border_fold     border gradients go to their source interior texels;
-//   k_blend_adjoint   G_k-1 (interior) = h G_k, g_x[r] = (1-h) sum_t w W^-1 G;
+//   k_blend_adjoint   border gradients go to their source interior texels,
+//                     G_k-1 (interior) = h G_k, g_x[r] = (1-h) sum_t w W^-1 G;
 //   k_ray_adjoint     g_x -> albedo, sun and sky gradients, and the two
 //                     sampleProbes lookups scatter into G_k-1 (atomics).
 // atlas_k-1 itself is restored from a checkpoint and replayed (k_replay_shade
@@ -67,30 +67,37 @@ __global__ void __launch_bounds__(128) k_replay_shade(DeviceScene sc, DeviceGrid
     rays[i] = rec;
 }
 
-// Adjoint of the border copy: a border texel's gradient belongs to the
-// interior texel it was copied from.
-__global__ void k_border_fold(DeviceGrid g, float4* gatlas) {
-    const uint32_t probe = blockIdx.x;
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)(g.res[0] * g.res[1]);
-    const int ix = (int)(probe % rx), iy = (int)((probe % rxy) / rx), iz = (int)(probe / rxy);
-    const int n = (int)g.color_res, tile = iy * g.res[0] + ix;
-    const int nb = 4 + 4 * (n - 2);
-    const size_t ox = (size_t)n * tile, oy = (size_t)n * iz;
-    for (int e = threadIdx.x; e < nb; e += blockDim.x) {
-        int4 b = border_entry(e, n);
-        float4* dst = gatlas + (oy + b.y) * g.color_w + ox + b.x;
-        float4* src = gatlas + (oy + b.w) * g.color_w + ox + b.z;
-        float4 v = *dst;
-        *dst = make_float4(0, 0, 0, 0);
-        atomicAdd(&src->x, v.x);
-        atomicAdd(&src->y, v.y);
-        atomicAdd(&src->z, v.z);
-    }
+// Gradient of an interior texel (sx, sy) of the tile at (ox, oy): its own and
+// those of the border texels that copy it (the inverse of border_entry).
+__device__ __forceinline__ float3 folded_gradient(const float4* __restrict__ g, size_t ox, size_t oy, uint32_t w, int n,
+                                                  int sx, int sy) {
+    const int e = n - 1, m = n - 2;
+    float3 s = f3(0, 0, 0);
+    auto take = [&](bool copied, int x, int y) {
+        if (!copied) return;
+        const float4 v = __ldg(g + (oy + y) * w + ox + x);
+        s = s + f3(v.x, v.y, v.z);
+    };
+    take(true, sx, sy);
+    take(sx == 1, 0, e - sy);
+    take(sx == m, e, e - sy);
+    take(sy == 1, e - sx, 0);
+    take(sy == m, e - sx, e);
+    take(sx == m && sy == m, 0, 0);
+    take(sx == m && sy == 1, 0, e);
+    take(sx == 1 && sy == m, e, 0);
+    take(sx == 1 && sy == 1, e, e);
+    return s;
 }
 
-// Adjoint of the colour blend + hysteresis of one probe (block = probe).
+// Adjoint of the colour blend + hysteresis + border copy of one probe (block =
+// probe).  wsum: the colour texels' weight sums, as the forward adds them up
+// (one launch for all probes; each block adding up its own, a chain of 256
+// loads by 36 threads, took 43 us for 2,048 probes of 256 rays, and a pass of
+// its own for the border 14 us; 17 us now and 7 us for the sums).
 __global__ void __launch_bounds__(256) k_blend_adjoint(DeviceGrid g, const float4* __restrict__ dirs,
-                                                       const float4* __restrict__ gk, float4* gprev, float4* gx) {
+                                                       const float* __restrict__ wsum, const float4* __restrict__ gk,
+                                                       float4* gprev, float4* gx) {
     extern __shared__ float smem[];
     const uint32_t R = g.rays;
     const int n = (int)g.color_res - 2, nt = n * n;
@@ -106,14 +113,10 @@ __global__ void __launch_bounds__(256) k_blend_adjoint(DeviceGrid g, const float
         int tx = t % n, ty = t / n;
         float sc = texel_scale((uint32_t)n), ce = 0.5f * (float)(n - 1);
         float3 td = oct_decode(sc * ((float)tx - ce), sc * ((float)ty - ce));
-        float W = 0.0f;
-        for (uint32_t r = 0; r < R; ++r) {  // ray order, as the forward sums it
-            float4 d = dirs[r];
-            W += fmaxf(0.0f, td.x * d.x + td.y * d.y + td.z * d.z);
-        }
+        const float W = wsum[t];
         float inv = W > 1e-3f ? 1.0f / W : 1.0f;
         size_t ti = (oy + 1 + ty) * g.color_w + ox + 1 + tx;
-        float4 gv = gk[ti];
+        const float3 gv = folded_gradient(gk, ox, oy, g.color_w, cres, 1 + tx, 1 + ty);
         gprev[ti] = make_float4(hy * gv.x, hy * gv.y, hy * gv.z, 0.0f);
         s_td[3 * t] = td.x;
         s_td[3 * t + 1] = td.y;
@@ -141,113 +144,111 @@ __global__ void __launch_bounds__(256) k_blend_adjoint(DeviceGrid g, const float
     }
 }
 
-// sampleProbes (irradiance.glsl:145-237) evaluated and differentiated with
-// respect to the colour atlas: returns the value, and adds
-// d(value)/d(texel) . gout into gatlas.  The weights depend only on geometry
-// and the depth atlas (constants here); d sqrt(c)/dc at c = 0 is taken as 0
-// (such texels receive only zero radiance whatever the parameters).
-__device__ float3 sample_probes_vjp(float3 position, float3 normal, float3 toCamera, const DeviceGrid& g,
-                                    const uint32_t* states, const AtlasF32& at, float3 gout, float4* gatlas) {
-    float3 cs = abs3(f3(g.cell[0], g.cell[1], g.cell[2]));
-    float3 gridCoords = (position - f3(g.mn[0], g.mn[1], g.mn[2])) / cs;
-    if (!(gridCoords.x >= 0.0f && gridCoords.y >= 0.0f && gridCoords.z >= 0.0f)) return f3(0, 0, 0);
-    float3 biasedPosition = position + (normal + toCamera) * g.bias;
-    int fx = (int)fminf(gridCoords.x, 16777216.0f), fy = (int)fminf(gridCoords.y, 16777216.0f),
-        fz = (int)fminf(gridCoords.z, 16777216.0f);
-    float3 alpha = (position - grid_probe_pos(g, fx, fy, fz)) / cs;
-    alpha = f3(clampf(alpha.x, 0.0f, 1.0f), clampf(alpha.y, 0.0f, 1.0f), clampf(alpha.z, 0.0f, 1.0f));
-    const float uvsx = (float)(g.res[0] * g.res[1]), uvsy = (float)g.res[2];
-    const float cr = (float)g.color_res, dr = (float)g.depth_res;
-    const float cscale = (float)(g.color_res - 2) / cr;
-    const float dscale = (float)(g.depth_res - 2) / dr;
-    const float2 nuv = sphere_to_oct_uv(normal);
-    float3 S = f3(0, 0, 0), Sf = f3(0, 0, 0);
-    float W = 0.0f, Wf = 0.0f;
-    // pass 0: sums; pass 1: scatter
-    for (int pass = 0; pass < 2; ++pass) {
-        float3 coef_f = f3(0, 0, 0), coef = f3(0, 0, 0);
-        if (pass == 1) {
-            float n = W > 1e-3f ? 1.0f / W : 1.0f, nf = Wf > 1e-3f ? 1.0f / Wf : 1.0f;
-            float a = 8.0f * clampf(W, 0.0f, 1.0f / 8.0f);
-            // d out / d s_i = (1-a) 2 Sf nf^2 wf_i + a 2 S n^2 w_i, per channel
-            coef_f = Sf * (2.0f * (1.0f - a) * nf * nf) * gout;
-            coef = S * (2.0f * a * n * n) * gout;
-        }
-#pragma unroll 1
-        for (int i = 0; i < 8; ++i) {
-            int ox = i & 1, oy = (i >> 1) & 1, oz = (i >> 2) & 1;
-            int px = fx + ox, py = fy + oy, pz = fz + oz;
-            if (px > g.res[0] - 1 || py > g.res[1] - 1 || pz > g.res[2] - 1) continue;
-            uint32_t lin = (uint32_t)(px + g.res[0] * py + g.res[0] * g.res[1] * pz);
-            if (__ldg(states + lin) == 0) continue;
-            float3 probePosition = grid_probe_pos(g, px, py, pz);
-            float3 directionToProbe = norm3(probePosition - position);
-            float3 biasedDirectionToProbe = probePosition - biasedPosition;
-            float2 duv = sphere_to_oct_uv(-norm3(biasedDirectionToProbe));
-            int tile = py * g.res[0] + px;
-            float cu = ((float)((int)g.color_res * tile + 1) / cr + cscale * nuv.x) / uvsx;
-            float cv = ((float)((int)g.color_res * pz + 1) / cr + cscale * nuv.y) / uvsy;
-            float du = ((float)((int)g.depth_res * tile + 1) / dr + dscale * duv.x) / uvsx;
-            float dv = ((float)((int)g.depth_res * pz + 1) / dr + dscale * duv.y) / uvsy;
-            float3 tri = f3(ox ? alpha.x : 1.0f - alpha.x, oy ? alpha.y : 1.0f - alpha.y, oz ? alpha.z : 1.0f - alpha.z);
-            float weight = 1.0f;
-            float bfw = fmaxf(0.0001f, (dot3(directionToProbe, normal) + 1.0f) * 0.5f);
-            weight *= bfw * bfw + 0.2f;
-            float fallbackWeight = weight;
-            float depth[2];
-            bilinear<2>(at.depth, g.depth_w, g.depth_h, du, dv, depth);
-            float mean = depth[0];
-            float variance = fabsf(depth[0] * depth[0] - depth[1]);
-            float dist = len3(probePosition - biasedPosition);
-            float dm = fmaxf(dist - mean, 0.0001f);
-            float cheb = variance / (variance + dm * dm);
-            cheb = fmaxf(cheb * cheb * cheb, 0.0f);
-            weight *= (dist <= mean) ? 1.0f : cheb;
-            weight = fmaxf(0.000001f, weight);
-            const float crush = 0.2f;
-            if (weight < crush) weight *= weight * weight * (1.0f / (crush * crush));
-            float triw = tri.x * tri.y * tri.z + 0.001f;
-            weight *= triw;
-            fallbackWeight *= triw;
-            // bilinear colour fetch (REPEAT) with its texel weights
-            float x = cu * (float)g.color_w - 0.5f, y = cv * (float)g.color_h - 0.5f;
-            float fx0 = floorf(x), fy0 = floorf(y);
-            float ax = x - fx0, ay = y - fy0;
-            int iw = (int)g.color_w, ih = (int)g.color_h;
-            int i0 = wrap_repeat((int)fx0, iw), i1 = wrap_repeat((int)fx0 + 1, iw);
-            int j0 = wrap_repeat((int)fy0, ih), j1 = wrap_repeat((int)fy0 + 1, ih);
-            size_t t00 = (size_t)j0 * g.color_w + i0, t10 = (size_t)j0 * g.color_w + i1;
-            size_t t01 = (size_t)j1 * g.color_w + i0, t11 = (size_t)j1 * g.color_w + i1;
-            float b00 = (1.0f - ax) * (1.0f - ay), b10 = ax * (1.0f - ay), b01 = (1.0f - ax) * ay, b11 = ax * ay;
-            float col[3];
-            bilinear<3>(at.color, g.color_w, g.color_h, cu, cv, col);
-            float3 s = f3(sqrtf(col[0]), sqrtf(col[1]), sqrtf(col[2]));
-            if (pass == 0) {
-                S = S + s * weight;
-                W += weight;
-                Sf = Sf + s * fallbackWeight;
-                Wf += fallbackWeight;
-            } else {
-                float3 ds = coef_f * fallbackWeight + coef * weight;  // dL/ds_i
-                float3 dc = f3(s.x > 0.0f ? ds.x / (2.0f * s.x) : 0.0f, s.y > 0.0f ? ds.y / (2.0f * s.y) : 0.0f,
-                               s.z > 0.0f ? ds.z / (2.0f * s.z) : 0.0f);
-                const size_t tt[4] = {t00, t10, t01, t11};
-                const float bw[4] = {b00, b10, b01, b11};
+// Adds (x, y, z, 0) to a texel's gradient: one 16-byte reduction.
+__device__ __forceinline__ void add_texel(float4* p, float x, float y, float z) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :
+                 : "l"(p), "f"(x), "f"(y), "f"(z), "f"(0.0f)
+                 : "memory");
+}
+
+constexpr int kAdjointThreads = 128;
+constexpr int kLookupWords = 32;  // weights of two lookups' eight probes, per thread in shared memory
+
+// The two lookups of a hit (sampleProbes, irradiance.glsl:145-237) evaluated
+// and differentiated with respect to the colour atlas: returns the values,
+// and adds d(value)/d(texel) . gout into gatlas.  The weights depend only on
+// geometry and the depth atlas (constants here); d sqrt(c)/dc at c = 0 is
+// taken as 0 (such texels receive only zero radiance whatever the parameters).
+//
+// The first pass over the eight probes is the forward's and keeps the weights
+// (`w`: this thread's column of kLookupWords in shared memory); the second
+// fetches the colours again and scatters.  Bound by the L2's reductions, 64 a
+// hit: of four floats each, where single floats took 192.  524 K rays of a
+// room: 580 us with both passes over everything, a lookup at a time, and
+// single-float reductions; 247 us now.
+__device__ __forceinline__ void sample_probes_vjp2(float3 position, const float3 (&normal)[2], float3 toCamera,
+                                                   const DeviceGrid& g, const uint32_t* states, const AtlasF32& at,
+                                                   const float3 (&gout)[2], float4* gatlas, float* w, float3 (&value)[2]) {
+    value[0] = value[1] = f3(0, 0, 0);
+    ProbeCell cell;
+    if (!probe_cell(position, g, states, &cell)) return;
+    const LookupScales s = lookup_scales(g);
+    float3 biased[2], S[2], Sf[2];
+    float2 nuv[2];
+    float W[2], Wf[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (bw[q] == 0.0f) continue;
-                    atomicAdd(&gatlas[tt[q]].x, dc.x * bw[q]);
-                    atomicAdd(&gatlas[tt[q]].y, dc.y * bw[q]);
-                    atomicAdd(&gatlas[tt[q]].z, dc.z * bw[q]);
-                }
-            }
+    for (int q = 0; q < 2; ++q) {
+        biased[q] = f3(fmaf(normal[q].x + toCamera.x, g.bias, position.x),
+                       fmaf(normal[q].y + toCamera.y, g.bias, position.y),
+                       fmaf(normal[q].z + toCamera.z, g.bias, position.z));
+        nuv[q] = oct_uv(normal[q]);
+        S[q] = Sf[q] = f3(0, 0, 0);
+        W[q] = Wf[q] = 0.0f;
+    }
+    // one lookup's colour at a probe, in square-root space, and its texels
+    auto colour = [&](const CellProbe& p, int q, Tap* t) {
+        *t = atlas_tap(p.tile + s.cinv, p.z + s.cinv, nuv[q], s.cscale, s.cr, g.color_w, g.color_h);
+        float c00[3], c10[3], c01[3], c11[3], r[3];
+        at.color.fetch(t->row0, c00);
+        at.color.fetch(t->row0 + 1u, c10);
+        at.color.fetch(t->row1, c01);
+        at.color.fetch(t->row1 + 1u, c11);
+        const float w11 = t->ax * t->ay, w10 = t->ax - w11, w01 = t->ay - w11, w00 = 1.0f - t->ax - w01;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r[k] = sqrtf(w00 * c00[k] + w10 * c10[k] + w01 * c01[k] + w11 * c11[k]);
+        return f3(r[0], r[1], r[2]);
+    };
+#pragma unroll 1
+    for (uint32_t live = cell.live; live != 0u; live &= live - 1u) {
+        const uint32_t i = (uint32_t)__ffs((int)live) - 1u;
+        const CellProbe p = cell_probe(cell, i, position, g);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            Tap t;
+            const float3 c = colour(p, q, &t);
+            float weight, fallback;
+            probe_weights(p, p.at - biased[q], normal[q], at.depth, s, g, &weight, &fallback);
+            w[(4 * i + 2 * q) * kAdjointThreads] = weight;
+            w[(4 * i + 2 * q + 1) * kAdjointThreads] = fallback;
+            S[q] = S[q] + c * weight;
+            W[q] += weight;
+            Sf[q] = Sf[q] + c * fallback;
+            Wf[q] += fallback;
         }
     }
-    float n = W > 1e-3f ? 1.0f / W : 1.0f, nf = Wf > 1e-3f ? 1.0f / Wf : 1.0f;
-    float3 fin = S * n, fb = Sf * nf;
-    fin = fin * fin;
-    fb = fb * fb;
-    return mix3(fb, fin, 8.0f * clampf(W, 0.0f, 1.0f / 8.0f));
+    float3 coef[2], coef_f[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const float n = W[q] > 1e-3f ? 1.0f / W[q] : 1.0f, nf = Wf[q] > 1e-3f ? 1.0f / Wf[q] : 1.0f;
+        const float a = 8.0f * clampf(W[q], 0.0f, 1.0f / 8.0f);
+        const float3 fin = S[q] * n, fb = Sf[q] * nf;
+        value[q] = mix3(fb * fb, fin * fin, a);
+        // d out / d s_i = (1-a) 2 Sf nf^2 wf_i + a 2 S n^2 w_i, per channel
+        coef_f[q] = fb * (2.0f * (1.0f - a) * nf) * gout[q];
+        coef[q] = fin * (2.0f * a * n) * gout[q];
+    }
+#pragma unroll 1
+    for (uint32_t live = cell.live; live != 0u; live &= live - 1u) {
+        const uint32_t i = (uint32_t)__ffs((int)live) - 1u;
+        const CellProbe p = cell_probe(cell, i, position, g);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            Tap t;
+            const float3 c = colour(p, q, &t);
+            const float weight = w[(4 * i + 2 * q) * kAdjointThreads], fallback = w[(4 * i + 2 * q + 1) * kAdjointThreads];
+            const float3 ds = coef_f[q] * fallback + coef[q] * weight;  // dL/ds_i
+            const float3 dc = f3(c.x > 0.0f ? ds.x / (2.0f * c.x) : 0.0f, c.y > 0.0f ? ds.y / (2.0f * c.y) : 0.0f,
+                                 c.z > 0.0f ? ds.z / (2.0f * c.z) : 0.0f);
+            const float w11 = t.ax * t.ay, w10 = t.ax - w11, w01 = t.ay - w11, w00 = 1.0f - t.ax - w01;
+            float4* p0 = gatlas + t.row0;
+            float4* p1 = gatlas + t.row1;
+            add_texel(p0, dc.x * w00, dc.y * w00, dc.z * w00);
+            if (w10 != 0.0f) add_texel(p0 + 1, dc.x * w10, dc.y * w10, dc.z * w10);
+            if (w01 != 0.0f) add_texel(p1, dc.x * w01, dc.y * w01, dc.z * w01);
+            if (w11 != 0.0f) add_texel(p1 + 1, dc.x * w11, dc.y * w11, dc.z * w11);
+        }
+    }
 }
 
 // Vector-Jacobian product of pbrMetallicRoughness with respect to albedo
@@ -296,13 +297,14 @@ __device__ float3 pbr_albedo_vjp(float3 n, float3 v, float3 lightColor, float3 l
 
 // Parameter gradients and the bounce scatter of every ray of one update.
 // grad layout (doubles): albedo [material_count][3], sun [3], sky [3].
-__global__ void __launch_bounds__(128) k_ray_adjoint(DeviceScene sc, DeviceGrid g, DeviceLight L,
+__global__ void __launch_bounds__(kAdjointThreads) k_ray_adjoint(DeviceScene sc, DeviceGrid g, DeviceLight L,
                                                      const float4* __restrict__ dirs,
                                                      const uint32_t* __restrict__ states, AtlasF32 at,
                                                      const float4* __restrict__ thit, const uint32_t* __restrict__ prim,
                                                      const float4* __restrict__ gx, float4* gatlas, double* grad,
                                                      uint32_t total, bool smem_albedo, uint32_t* err) {
     extern __shared__ double s_grad[];  // [M*3 if smem_albedo] + sun[3] + sky[3]
+    __shared__ float s_weights[kLookupWords][kAdjointThreads];
     const uint32_t M3 = smem_albedo ? sc.material_count * 3 : 0;
     for (uint32_t k = threadIdx.x; k < M3 + 6; k += blockDim.x) s_grad[k] = 0.0;
     __syncthreads();
@@ -333,8 +335,11 @@ __global__ void __launch_bounds__(128) k_ray_adjoint(DeviceScene sc, DeviceGrid 
                 float3 g_base = shadowed ? gxi : gxi * fade;
                 float3 g_pbr = shadowed ? f3(0, 0, 0) : gxi * fade;
                 float3 reflectDir = dir - s.normal * (2.0f * dot3(s.normal, dir));
-                float3 refl = sample_probes_vjp(s.position, reflectDir, -dir, g, states, at, g_base * spec, gatlas);
-                float3 ind = sample_probes_vjp(s.position, s.normal, -dir, g, states, at, g_base * diffuse, gatlas);
+                const float3 lookups[2] = {reflectDir, s.normal}, gout[2] = {g_base * spec, g_base * diffuse};
+                float3 value[2];  // reflection, indirect
+                sample_probes_vjp2(s.position, lookups, -dir, g, states, at, gout, gatlas, &s_weights[0][threadIdx.x],
+                                   value);
+                const float3 refl = value[0], ind = value[1];
                 float3 ga = g_base * (refl * s.metal + ind * ((1.0f - 0.04f) * (1.0f - s.metal)));
                 if (!shadowed) {
                     float3 v = norm3(-dir);
@@ -377,17 +382,18 @@ cudaError_t launch_replay_update(const DeviceScene& sc, const DeviceGrid& g, con
 
 cudaError_t launch_adjoint_step(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L, const float4* dirs,
                                 const uint32_t* states, const float4* color_prev, const float2* depth_prev,
-                                const float4* thit, const uint32_t* prim, float4* gk, float4* gprev, float4* gx,
-                                double* grad, uint32_t* err, cudaStream_t st) {
+                                const float4* thit, const uint32_t* prim, const float4* gk, float4* gprev, float4* gx,
+                                float* W, float* wsum, double* grad, uint32_t* err, cudaStream_t st) {
     const uint32_t P = (uint32_t)(g.res[0] * g.res[1] * g.res[2]);
     const uint32_t total = P * g.rays;
-    k_border_fold<<<P, 64, 0, st>>>(g, gk);
     const uint32_t nt = (g.color_res - 2) * (g.color_res - 2);
-    k_blend_adjoint<<<P, 256, sizeof(float) * 6 * nt, st>>>(g, dirs, gk, gprev, gx);
+    cudaError_t e = launch_color_weights(g, dirs, W, wsum, st);
+    if (e != cudaSuccess) return e;
+    k_blend_adjoint<<<P, 256, sizeof(float) * 6 * nt, st>>>(g, dirs, wsum, gk, gprev, gx);
     AtlasF32 at{{color_prev}, {depth_prev}};
     const bool smem_albedo = sc.material_count <= 1024;
     size_t smem = sizeof(double) * ((smem_albedo ? sc.material_count * 3 : 0) + 6);
-    k_ray_adjoint<<<(total + 127) / 128, 128, smem, st>>>(sc, g, L, dirs, states, at, thit, prim, gx, gprev, grad,
+    k_ray_adjoint<<<(total + kAdjointThreads - 1) / kAdjointThreads, kAdjointThreads, smem, st>>>(sc, g, L, dirs, states, at, thit, prim, gx, gprev, grad,
                                                           total, smem_albedo, err);
     return cudaGetLastError();
 }

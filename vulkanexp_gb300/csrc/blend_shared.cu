@@ -375,6 +375,13 @@ cudaError_t set_shared_smem_limit() {
     return e;
 }
 
+cudaError_t launch_color_weights(const DeviceGrid& g, const float4* dirs, float* W, float* wsum, cudaStream_t st) {
+    // the colour texels come first; a last block's depth texels do no harm
+    k_fp32_weights<<<weight_blocks((g.color_res - 2) * (g.color_res - 2)), 256, weight_smem(g.rays), st>>>(g, dirs, W,
+                                                                                                         wsum);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_blend_fp32_shared(const DeviceGrid& g, const uint32_t* probe_list, uint32_t nprobes,
                                      const float4* rays, const float4* dirs, float* W, float* wsum, uint32_t* states,
                                      float4* color, float2* depth, cudaStream_t st, const uint32_t* dev_count,

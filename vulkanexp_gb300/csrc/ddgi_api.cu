@@ -2280,7 +2280,7 @@ ddgi_status ddgi_backward(ddgi_ctx* ctx, const float* dL_dcolor, size_t bytes, f
         if (s != DDGI_OK) return s;
         CK(launch_adjoint_step(sc, ctx->dg, ctx->dl, ctx->dirs, ctx->work_states, ctx->work_color, ctx->work_depth,
                                ctx->rec_thit + rays * u, ctx->rec_prim + rays * u, ctx->g_a, ctx->g_b, ctx->g_x,
-                               ctx->d_grad, ctx->err, st),
+                               reinterpret_cast<float*>(ctx->tc_weights), ctx->tc_rowsum, ctx->d_grad, ctx->err, st),
            "adjoint");
         std::swap(ctx->g_a, ctx->g_b);
     }

@@ -198,8 +198,8 @@ cudaError_t launch_replay_update(const DeviceScene& sc, const DeviceGrid& g, con
                                  cudaStream_t st);
 cudaError_t launch_adjoint_step(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L, const float4* dirs,
                                 const uint32_t* states, const float4* color_prev, const float2* depth_prev,
-                                const float4* thit, const uint32_t* prim, float4* gk, float4* gprev, float4* gx,
-                                double* grad, uint32_t* err, cudaStream_t st);
+                                const float4* thit, const uint32_t* prim, const float4* gk, float4* gprev, float4* gx,
+                                float* W, float* wsum, double* grad, uint32_t* err, cudaStream_t st);
 
 // blend_tc.cu
 size_t tc_weight_bytes(uint32_t rays, uint32_t color_res, uint32_t depth_res);
@@ -214,6 +214,8 @@ cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uin
 size_t fp32_weight_bytes(uint32_t rays, uint32_t color_res, uint32_t depth_res);
 uint32_t fp32_shared_tiles(uint32_t nprobes);
 cudaError_t set_shared_smem_limit();  // both shared-weight FP32 blend kernels, current device
+// the colour texels' weights and sums alone (wsum[0 .. (color_res - 2)^2))
+cudaError_t launch_color_weights(const DeviceGrid& g, const float4* dirs, float* W, float* wsum, cudaStream_t st);
 cudaError_t launch_blend_fp32_shared(const DeviceGrid& g, const uint32_t* probe_list, uint32_t nprobes,
                                      const float4* rays, const float4* dirs, float* W, float* wsum, uint32_t* states,
                                      float4* color, float2* depth, cudaStream_t st, const uint32_t* dev_count = nullptr,
