@@ -56,10 +56,61 @@ DDGI_HD static inline float ts_div(float a, float b) {
     return a / b;
 #endif
 }
-DDGI_HD static inline float ts_down(float x) { return nextafterf(x, -INFINITY); }
-DDGI_HD static inline float ts_up(float x) { return nextafterf(x, INFINITY); }
-DDGI_HD static inline float ts_min4(float a, float b, float c, float d) { return fminf(fminf(a, b), fminf(c, d)); }
-DDGI_HD static inline float ts_max4(float a, float b, float c, float d) { return fmaxf(fmaxf(a, b), fmaxf(c, d)); }
+// The neighbouring float above / below x.  Floats of one sign are ordered as
+// their bit patterns are, so on the device the neighbour is the pattern one
+// away (+0 stands for both zeros; +infinity and NaN stay): nextafterf's value
+// in six instructions.
+DDGI_HD static inline float ts_up(float x) {
+#ifdef __CUDA_ARCH__
+    const int i = __float_as_int(__fadd_rn(x, 0.0f));
+    return x < INFINITY ? __int_as_float(i + ((i >> 31) | 1)) : x;
+#else
+    return nextafterf(x, INFINITY);
+#endif
+}
+DDGI_HD static inline float ts_down(float x) {
+#ifdef __CUDA_ARCH__
+    return -ts_up(-x);
+#else
+    return nextafterf(x, -INFINITY);
+#endif
+}
+
+DDGI_HD static inline bool ts_crosses(float p, float q, float pl) { return (p < pl && q > pl) || (p > pl && q < pl); }
+
+// The crossing of edge p -> q with the plane x_K = pl, strictly between p and
+// q, added to the bounds of both sides.  t = (pl - p_K) / (q_K - p_K) lies in
+// (0, 1); numerator and denominator have the same sign, and rounding is
+// monotonic, so of the four quotients of their intervals' ends the lowest is
+// that of the smallest numerator and the largest denominator and the highest
+// the other way round (magnitudes), and of the four products of (q_a - p_a)
+// and t, t >= 0, the signs tell the lowest and the highest.
+template <int K>
+DDGI_HD static inline void ts_crossing(const float* p, const float* q, float pl, float llo[3], float lhi[3],
+                                       float glo[3], float ghi[3]) {
+    const float n = ts_sub(pl, p[K]), d = ts_sub(q[K], p[K]);
+    const float dlo = ts_down(d), dhi = ts_up(d);
+    float t0 = 0.0f, t1 = 1.0f;
+    if (dlo > 0.0f || dhi < 0.0f) {
+        const float nlo = ts_down(n), nhi = ts_up(n);
+        const bool up = dlo > 0.0f;
+        t0 = fmaxf(0.0f, ts_down(ts_div(up ? nlo : nhi, up ? dhi : dlo)));
+        t1 = fminf(1.0f, ts_up(ts_div(up ? nhi : nlo, up ? dlo : dhi)));
+    }
+    for (int a = 0; a < 3; ++a) {
+        float clo = pl, chi = pl;  // the crossing's own axis is the plane exactly
+        if (a != K) {
+            const float dd = ts_sub(q[a], p[a]);
+            const float ddlo = ts_down(dd), ddhi = ts_up(dd);
+            clo = ts_down(ts_add(p[a], ts_down(ts_mul(ddlo, ddlo >= 0.0f ? t0 : t1))));
+            chi = ts_up(ts_add(p[a], ts_up(ts_mul(ddhi, ddhi >= 0.0f ? t1 : t0))));
+        }
+        llo[a] = fminf(llo[a], clo);
+        lhi[a] = fmaxf(lhi[a], chi);
+        glo[a] = fminf(glo[a], clo);
+        ghi[a] = fmaxf(ghi[a], chi);
+    }
+}
 
 // Bounds of the parts of triangle `tri` (9 floats: v0, v1, v2) on either
 // side of the plane x_K = pl: below (x_K <= pl) into llo/lhi, above
@@ -86,34 +137,18 @@ DDGI_HD static inline void tri_plane_bounds_k(const float* tri, float pl, float 
                 ghi[a] = fmaxf(ghi[a], p[a]);
             }
     }
-    for (int e = 0; e < 3; ++e) {
-        const float* p = tri + 3 * e;
-        const float* q = tri + 3 * (e == 2 ? 0 : e + 1);
-        if (!((p[K] < pl && q[K] > pl) || (p[K] > pl && q[K] < pl))) continue;
-        // t = (pl - p_K) / (q_K - p_K), in (0, 1) exactly
-        const float n = ts_sub(pl, p[K]), d = ts_sub(q[K], p[K]);
-        const float nlo = ts_down(n), nhi = ts_up(n), dlo = ts_down(d), dhi = ts_up(d);
-        float t0 = 0.0f, t1 = 1.0f;
-        if (dlo > 0.0f || dhi < 0.0f) {
-            const float c0 = ts_div(nlo, dlo), c1 = ts_div(nlo, dhi), c2 = ts_div(nhi, dlo), c3 = ts_div(nhi, dhi);
-            t0 = fmaxf(0.0f, ts_down(ts_min4(c0, c1, c2, c3)));
-            t1 = fminf(1.0f, ts_up(ts_max4(c0, c1, c2, c3)));
-        }
-        for (int a = 0; a < 3; ++a) {
-            float clo = pl, chi = pl;  // the crossing's own axis is the plane exactly
-            if (a != K) {
-                const float dd = ts_sub(q[a], p[a]);
-                const float ddlo = ts_down(dd), ddhi = ts_up(dd);
-                const float m0 = ts_mul(ddlo, t0), m1 = ts_mul(ddlo, t1), m2 = ts_mul(ddhi, t0), m3 = ts_mul(ddhi, t1);
-                clo = ts_down(ts_add(p[a], ts_down(ts_min4(m0, m1, m2, m3))));
-                chi = ts_up(ts_add(p[a], ts_up(ts_max4(m0, m1, m2, m3))));
-            }
-            llo[a] = fminf(llo[a], clo);
-            lhi[a] = fmaxf(lhi[a], chi);
-            glo[a] = fminf(glo[a], clo);
-            ghi[a] = fmaxf(ghi[a], chi);
-        }
+    // at most two edges cross: those of the vertex alone on its side
+    const bool c0 = ts_crosses(tri[K], tri[3 + K], pl), c1 = ts_crosses(tri[3 + K], tri[6 + K], pl),
+               c2 = ts_crosses(tri[6 + K], tri[K], pl);
+    const int v = c0 ? (c1 ? 1 : 0) : (c1 && !c2 ? 1 : 2);
+    float at[3], next[3], before[3];
+    for (int a = 0; a < 3; ++a) {
+        at[a] = v == 0 ? tri[a] : (v == 1 ? tri[3 + a] : tri[6 + a]);
+        next[a] = v == 0 ? tri[3 + a] : (v == 1 ? tri[6 + a] : tri[a]);
+        before[a] = v == 0 ? tri[6 + a] : (v == 1 ? tri[a] : tri[3 + a]);
     }
+    if (v == 0 ? c0 : (v == 1 ? c1 : c2)) ts_crossing<K>(at, next, pl, llo, lhi, glo, ghi);
+    if (v == 0 ? c2 : (v == 1 ? c0 : c1)) ts_crossing<K>(before, at, pl, llo, lhi, glo, ghi);
 }
 
 DDGI_HD static inline void tri_plane_bounds(const float* tri, int k, float pl, float llo[3], float lhi[3], float glo[3],
