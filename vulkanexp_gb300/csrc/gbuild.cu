@@ -75,13 +75,16 @@ constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kMaxSplitDepth = 40;  // sbvh.cu: no spatial split below this depth
 constexpr uint32_t kSweepMax = 4096;     // sah.cu: exact sweep at or below this many references
 constexpr int kSweepThreads = 512;
+// Mesh-tree nodes of at most this many references are split by one warp each,
+// two references a lane (k_small).
+constexpr uint32_t kSmallNode = 64;
 constexpr int kObjWords = 7;   // count, lo keys xyz, hi keys xyz
 constexpr int kSpWords = 8;    // enter, leave, lo keys xyz, hi keys xyz
 constexpr int kBinWords = 3 * kBins * (kObjWords + kSpWords);
 constexpr uint32_t kKeyPosInf = 0xFF800000u, kKeyNegInf = 0x007FFFFFu;
 
 enum Kind : int32_t { kObject = 0, kSpatial = 1, kHalve = 2 };
-enum Ctr : int { kCtrNodes = 0, kCtrRefs, kCtrChunks, kCtrBins, kCtrPool, kCtrOverflow, kCtrSweep, kCtrs = 8 };
+enum Ctr : int { kCtrNodes = 0, kCtrRefs, kCtrChunks, kCtrBins, kCtrPool, kCtrOverflow, kCtrSweep, kCtrSmall, kCtrs = 8 };
 
 struct Ref {
     float4 lo, hi;  // box; lo.w holds the primitive (global index) as bits
@@ -148,6 +151,9 @@ __device__ __forceinline__ float centroid(const DBox& b, int k) {
     const float c = __fmul_rn(0.5f, __fadd_rn(b.lo[k], b.hi[k]));
     return c == c ? c : -INFINITY;
 }
+__device__ __forceinline__ float centroid_at(const DBox& b, int k) {
+    return k == 0 ? centroid(b, 0) : (k == 1 ? centroid(b, 1) : centroid(b, 2));
+}
 __device__ __forceinline__ int bin_of(float x, float lo, float scale) {
     const float f = __fmul_rn(__fsub_rn(x, lo), scale);
     if (!(f >= 0.0f)) return 0;
@@ -182,6 +188,30 @@ __device__ __forceinline__ void box_clip(DBox& b, const DBox& o) {
     for (int k = 0; k < 3; ++k) {
         b.lo[k] = fmaxf(b.lo[k], o.lo[k]);
         b.hi[k] = fminf(b.hi[k], o.hi[k]);
+    }
+}
+
+// tri_plane_bounds of axis k with the axes rotated so that k comes first: one
+// body for the three axes (the axes' operations are independent of each
+// other), a third of the instructions to fetch and no branch between lanes
+// that cut along different axes.
+__device__ __forceinline__ float pick3(int k, float a, float b, float c) { return k == 0 ? a : (k == 1 ? b : c); }
+__device__ __forceinline__ void tri_plane_boxes(const float* tri, int k, float pl, DBox& below, DBox& above) {
+    float t[9], blo[3], bhi[3], alo[3], ahi[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        t[3 * v] = pick3(k, tri[3 * v], tri[3 * v + 1], tri[3 * v + 2]);
+        t[3 * v + 1] = pick3(k, tri[3 * v + 1], tri[3 * v + 2], tri[3 * v]);
+        t[3 * v + 2] = pick3(k, tri[3 * v + 2], tri[3 * v], tri[3 * v + 1]);
+    }
+    tri_plane_bounds_k<0>(t, pl, blo, bhi, alo, ahi);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {  // axis a is rotated axis (a - k) mod 3
+        const int i = a, j = (a + 2) % 3, l = (a + 1) % 3;
+        below.lo[a] = pick3(k, blo[i], blo[j], blo[l]);
+        below.hi[a] = pick3(k, bhi[i], bhi[j], bhi[l]);
+        above.lo[a] = pick3(k, alo[i], alo[j], alo[l]);
+        above.hi[a] = pick3(k, ahi[i], ahi[j], ahi[l]);
     }
 }
 
@@ -286,6 +316,8 @@ struct Pass {
     uint32_t* bins_out;          // next level's
     const uint32_t* sweep_in;    // this level's swept nodes (box sets)
     uint32_t* sweep_out;
+    const uint32_t* small_in;    // this level's small nodes (triangle sets)
+    uint32_t* small_out;
     uint32_t* pool;              // leaf references (primitive, global index)
     uint32_t* ctr;
     uint32_t cap_refs, cap_chunks, cap_bins;
@@ -396,7 +428,14 @@ __global__ void __launch_bounds__(kThreads) k_init_refs(Pass P, Ref* refs, const
 // ---------------------------------------------------------------------------
 // Object split
 // ---------------------------------------------------------------------------
-__device__ void eval_object(const Pass& P, BNode& N, const uint32_t* s_bin, const float* s_scale) {
+struct ObjectSplit {
+    float cost;
+    int axis, plane;  // axis -1: none
+    bool spatial;     // the children overlap enough to try spatial splits
+};
+// By one warp, from the node's object bins; the same in every lane.
+__device__ __forceinline__ ObjectSplit eval_object(const Pass& P, const BNode& N, const uint32_t* s_bin,
+                                                   const float* s_scale) {
     const int lane = threadIdx.x & 31;
     const uint32_t n = N.count;
     float best = INFINITY;
@@ -404,6 +443,7 @@ __device__ void eval_object(const Pass& P, BNode& N, const uint32_t* s_bin, cons
     DBox bl, br;
     box_reset(bl);
     box_reset(br);
+#pragma unroll 1
     for (int k = 0; k < 3; ++k) {
         if (s_scale[k] == 0.0f) continue;
         const uint32_t* q = s_bin + kObjWords * (k * kBins + lane);
@@ -437,14 +477,27 @@ __device__ void eval_object(const Pass& P, BNode& N, const uint32_t* s_bin, cons
         const float root_area = half_area(key_box(P.nodes[P.set_root[N.set]].nb));
         spatial = half_area(ov) > __fmul_rn(P.alpha, root_area);
     }
-    if (lane == 0) {
-        N.oax = bax;
-        N.oplane = bplane;
-        N.ocost = best;
-        N.spatial = spatial ? 1u : 0u;
-        N.kind = bax >= 0 ? kObject : kHalve;
-        N.sax = -1;
+    return ObjectSplit{best, bax, bplane, spatial};
+}
+
+// Adds a reference to the object bins.
+__device__ __forceinline__ void bin_object(uint32_t* s_bin, const DBox& b, const float* s_clo, const float* s_scale) {
+    for (int k = 0; k < 3; ++k) {
+        if (s_scale[k] == 0.0f) continue;
+        uint32_t* q = s_bin + kObjWords * (k * kBins + bin_of(centroid(b, k), s_clo[k], s_scale[k]));
+        atomicAdd(q, 1u);
+        for (int a = 0; a < 3; ++a) {
+            atomicMin(q + 1 + a, fkey(b.lo[a]));
+            atomicMax(q + 4 + a, fkey(b.hi[a]));
+        }
     }
+}
+
+// The centroid grid of an axis; scale 0: the axis is skipped.
+__device__ __forceinline__ void object_axis(const BNode& N, int k, float* lo, float* scale) {
+    *lo = kval(N.cb[k]);
+    const float ext = __fsub_rn(kval(N.cb[3 + k]), *lo);
+    *scale = ext > 0.0f && ext < INFINITY ? __fdiv_rn((float)kBins, ext) : 0.0f;
 }
 
 __global__ void __launch_bounds__(kThreads) k_bin_object(Pass P) {
@@ -454,33 +507,26 @@ __global__ void __launch_bounds__(kThreads) k_bin_object(Pass P) {
     const uint32_t c = blockIdx.x;
     BNode& N = P.nodes[P.chunk_node[c]];
     for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) init_bin_words(s_bin + kObjWords * i, kObjWords);
-    if (threadIdx.x < 3) {
-        const int k = threadIdx.x;
-        const float lo = kval(N.cb[k]), hi = kval(N.cb[3 + k]);
-        const float ext = __fsub_rn(hi, lo);
-        s_clo[k] = lo;
-        s_scale[k] = ext > 0.0f && ext < INFINITY ? __fdiv_rn((float)kBins, ext) : 0.0f;  // 0: axis skipped
-    }
+    if (threadIdx.x < 3) object_axis(N, threadIdx.x, &s_clo[threadIdx.x], &s_scale[threadIdx.x]);
     __syncthreads();
     uint32_t p0, p1;
     chunk_range(N, c, p0, p1);
-    for (uint32_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-        const DBox b = ref_box(P.in[p]);
-        for (int k = 0; k < 3; ++k) {
-            if (s_scale[k] == 0.0f) continue;
-            uint32_t* q = s_bin + kObjWords * (k * kBins + bin_of(centroid(b, k), s_clo[k], s_scale[k]));
-            atomicAdd(q, 1u);
-            for (int a = 0; a < 3; ++a) {
-                atomicMin(q + 1 + a, fkey(b.lo[a]));
-                atomicMax(q + 4 + a, fkey(b.hi[a]));
-            }
-        }
-    }
+    for (uint32_t p = p0 + threadIdx.x; p < p1; p += blockDim.x)
+        bin_object(s_bin, ref_box(P.in[p]), s_clo, s_scale);
     __syncthreads();
     if (N.nchunks > 1 &&
         !merge_bins(s_bin, P.bins + (size_t)N.bins * kBinWords, 3 * kBins, kObjWords, &N.ctr[0], N.nchunks, &s_last))
         return;
-    if (threadIdx.x < 32) eval_object(P, N, s_bin, s_scale);
+    if (threadIdx.x >= 32) return;
+    const ObjectSplit o = eval_object(P, N, s_bin, s_scale);
+    if (threadIdx.x == 0) {
+        N.oax = o.axis;
+        N.oplane = o.plane;
+        N.ocost = o.cost;
+        N.spatial = o.spatial ? 1u : 0u;
+        N.kind = o.axis >= 0 ? kObject : kHalve;
+        N.sax = -1;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -497,149 +543,53 @@ __device__ __forceinline__ void grow_bin(uint32_t* q, const DBox& b) {
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_bin_spatial(Pass P) {
-    __shared__ uint32_t s_bin[3 * kBins * kSpWords];
-    __shared__ float s_lo[3], s_hi[3], s_w[3], s_scale[3];
-    __shared__ uint32_t s_cnt[3 * kThreads], s_off[3 * kThreads], s_total;
-    __shared__ uint8_t s_b0[3 * kThreads];
-    __shared__ float s_above[kThreads][6];
-    __shared__ float s_carry[6];
-    __shared__ int s_last;
-    const uint32_t c = blockIdx.x;
-    BNode& N = P.nodes[P.chunk_node[c]];
-    if (!N.spatial) return;  // the whole block
-    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) init_bin_words(s_bin + kSpWords * i, kSpWords);
-    if (threadIdx.x < 3) {
-        const int k = threadIdx.x;
-        const float lo = kval(N.nb[k]), hi = kval(N.nb[3 + k]);
-        const float ext = __fsub_rn(hi, lo);
-        const bool ok = ext > 0.0f && ext < INFINITY;
-        s_lo[k] = lo;
-        s_hi[k] = hi;
-        s_w[k] = ok ? __fdiv_rn(ext, (float)kBins) : 0.0f;
-        s_scale[k] = ok ? __fdiv_rn((float)kBins, ext) : 0.0f;
+// The bin planes of an axis; scale 0: the axis is skipped.
+__device__ __forceinline__ void spatial_axis(const BNode& N, int k, float* lo, float* hi, float* w, float* scale) {
+    *lo = kval(N.nb[k]);
+    *hi = kval(N.nb[3 + k]);
+    const float ext = __fsub_rn(*hi, *lo);
+    const bool ok = ext > 0.0f && ext < INFINITY;
+    *w = ok ? __fdiv_rn(ext, (float)kBins) : 0.0f;
+    *scale = ok ? __fdiv_rn((float)kBins, ext) : 0.0f;
+}
+
+// A reference's first and last bin along axis k counted (and, when they are
+// one, its box added); returns the planes between them, *first the first bin.
+__device__ __forceinline__ uint32_t bin_spatial_ends(uint32_t* s_bin, const DBox& rb, int k, float lo, float scale,
+                                                     int* first) {
+    const int b0 = bin_of(rb.lo[k], lo, scale);
+    const int b1 = max(b0, bin_of(rb.hi[k], lo, scale));
+    uint32_t* sb = s_bin + kSpWords * kBins * k;
+    atomicAdd(sb + kSpWords * b0, 1u);
+    atomicAdd(sb + kSpWords * b1 + 1, 1u);
+    if (b0 == b1) grow_bin(sb + kSpWords * b0 + 2, rb);
+    *first = b0;
+    return (uint32_t)(b1 - b0);
+}
+
+// One inner plane of a reference spanning bins first .. : bin `bin` gets the
+// part below the plane and above the previous one, the bin after the last
+// plane the part above it.
+__device__ __forceinline__ void bin_spatial_part(uint32_t* s_bin, int k, int bin, const DBox& rb, bool first, bool last,
+                                                 const DBox& prev, const DBox& below, const DBox& above) {
+    uint32_t* sb = s_bin + kSpWords * kBins * k;
+    DBox part = rb;
+    if (!first) box_clip(part, prev);
+    box_clip(part, below);
+    if (!box_empty(part)) grow_bin(sb + kSpWords * bin + 2, part);
+    if (last) {
+        DBox tail = rb;
+        box_clip(tail, above);
+        if (!box_empty(tail)) grow_bin(sb + kSpWords * (bin + 1) + 2, tail);
     }
-    __syncthreads();
-    uint32_t p0, p1;
-    chunk_range(N, c, p0, p1);
-    // Rounds of kThreads references.  A reference spanning bins b0 < b1
-    // along axis k has the m = b1 - b0 inner bin planes p_(b0+1) .. p_(b1);
-    // the (reference, axis, plane) triples of a round are numbered
-    // axis-major and dealt out one per thread, each thread computing the
-    // triangle's bounds below and above its plane (tri_split.h).  Bin
-    // b0 + i then gets the reference's box cut to "below plane i" and
-    // "above plane i - 1" (the previous triple, the neighbouring thread or
-    // the previous sub-round's last one), bin b1 the box cut to "above plane
-    // m - 1": sbvh.cu's binning, dealt out evenly.
-    for (uint32_t r0 = p0; r0 < p1; r0 += kThreads) {
-        const uint32_t nr = min((uint32_t)kThreads, p1 - r0);
-        __syncthreads();  // the previous round's tables are read
-        {
-            const uint32_t t = threadIdx.x;
-            for (int k = 0; k < 3; ++k) {
-                uint32_t m = 0;
-                int b0 = 0;
-                if (t < nr && s_scale[k] != 0.0f) {
-                    const DBox rb = ref_box(P.in[r0 + t]);
-                    b0 = bin_of(rb.lo[k], s_lo[k], s_scale[k]);
-                    const int b1 = max(b0, bin_of(rb.hi[k], s_lo[k], s_scale[k]));
-                    uint32_t* sb = s_bin + kSpWords * kBins * k;
-                    atomicAdd(sb + kSpWords * b0, 1u);
-                    atomicAdd(sb + kSpWords * b1 + 1, 1u);
-                    if (b0 == b1) grow_bin(sb + kSpWords * b0 + 2, rb);
-                    m = (uint32_t)(b1 - b0);
-                }
-                s_cnt[k * kThreads + t] = m;
-                s_b0[k * kThreads + t] = (uint8_t)b0;
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) {  // exclusive scan of the 3 x kThreads plane counts
-            uint32_t run = 0;
-            for (int base = 0; base < 3 * kThreads; base += 32) {
-                const uint32_t v = s_cnt[base + threadIdx.x];
-                uint32_t x = v;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                    if ((int)threadIdx.x >= o) x += y;
-                }
-                s_off[base + threadIdx.x] = run + x - v;
-                run += __shfl_sync(0xFFFFFFFFu, x, 31);
-            }
-            if (threadIdx.x == 0) s_total = run;
-        }
-        __syncthreads();
-        const uint32_t total = s_total;
-        for (uint32_t g0 = 0; g0 < total; g0 += kThreads) {
-            const uint32_t g = g0 + threadIdx.x;
-            DBox below, above, rb;
-            int bin = -1, k = 0;
-            bool last = false;
-            uint32_t i = 0;
-            if (g < total) {
-                // the triple holding plane g: the last entry with s_off <= g
-                int lo = 0, hi = 3 * kThreads - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_off[mid] <= g) lo = mid;
-                    else hi = mid - 1;
-                }
-                // (an entry without planes shares its offset with the next
-                // one, so the last entry at or below g has planes)
-                k = lo / kThreads;
-                const uint32_t t = (uint32_t)(lo % kThreads);
-                i = g - s_off[lo];
-                last = i + 1 == s_cnt[lo];
-                const int b0 = s_b0[lo];
-                bin = b0 + (int)i;
-                const Ref r = P.in[r0 + t];
-                rb = ref_box(r);
-                float tri[9];
-                load_tri(P.tris + 9 * (size_t)ref_prim(r), tri);
-                const float pl = plane_at(s_lo[k], s_hi[k], s_w[k], bin + 1);
-                if (k == 0) tri_plane_bounds_k<0>(tri, pl, below.lo, below.hi, above.lo, above.hi);
-                else if (k == 1) tri_plane_bounds_k<1>(tri, pl, below.lo, below.hi, above.lo, above.hi);
-                else tri_plane_bounds_k<2>(tri, pl, below.lo, below.hi, above.lo, above.hi);
-                for (int a = 0; a < 3; ++a) {
-                    s_above[threadIdx.x][a] = above.lo[a];
-                    s_above[threadIdx.x][3 + a] = above.hi[a];
-                }
-            }
-            __syncthreads();
-            DBox prev;
-            if (g < total && i > 0) {
-                const float* q = threadIdx.x > 0 ? s_above[threadIdx.x - 1] : s_carry;
-                for (int a = 0; a < 3; ++a) {
-                    prev.lo[a] = q[a];
-                    prev.hi[a] = q[3 + a];
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == kThreads - 1)
-                for (int a = 0; a < 6; ++a) s_carry[a] = s_above[kThreads - 1][a];
-            if (g < total) {
-                uint32_t* sb = s_bin + kSpWords * kBins * k;
-                DBox part = rb;
-                if (i > 0) box_clip(part, prev);
-                box_clip(part, below);
-                if (!box_empty(part)) grow_bin(sb + kSpWords * bin + 2, part);
-                if (last) {
-                    DBox tail = rb;
-                    box_clip(tail, above);
-                    if (!box_empty(tail)) grow_bin(sb + kSpWords * (bin + 1) + 2, tail);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (N.nchunks > 1 && !merge_bins(s_bin, P.bins + (size_t)N.bins * kBinWords + 3 * kBins * kObjWords, 3 * kBins,
-                                     kSpWords, &N.ctr[1], N.nchunks, &s_last))
-        return;
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    float best = N.ocost;
+}
+
+// By one warp, from the node's spatial bins: the axis of the best plane
+// cheaper than `best` (-1: none) and its bin; the same in every lane.
+__device__ __forceinline__ int eval_spatial(const uint32_t* s_bin, const float* s_scale, float best, int* plane) {
+    const int lane = threadIdx.x & 31;
     int sax = -1;
-    float splane = 0.0f;
+#pragma unroll 1
     for (int k = 0; k < 3; ++k) {
         if (s_scale[k] == 0.0f) continue;
         const uint32_t* q = s_bin + kSpWords * (k * kBins + lane);
@@ -656,13 +606,127 @@ __global__ void __launch_bounds__(kThreads) k_bin_spatial(Pass P) {
         if (m < best) {
             best = m;
             sax = k;
-            splane = plane_at(s_lo[k], s_hi[k], s_w[k], j);
+            *plane = j;
         }
     }
-    if (lane == 0 && sax >= 0) {
+    return sax;
+}
+
+// Bin planes of a node's axes, in shared memory.
+struct SpatialGrid {
+    float lo[3], hi[3], w[3], scale[3];
+};
+// One round's (reference, axis) entries, per warp in shared memory.
+struct RoundTable {
+    uint32_t cnt[3 * 32], off[3 * 32];
+    uint8_t b0[3 * 32];
+};
+
+// References p0 .. p1 - 1 added to the spatial bins by one warp, in rounds of
+// 32 references `stride` apart.  A reference spanning bins b0 < b1 along axis
+// k has the m = b1 - b0 inner bin planes p_(b0+1) .. p_(b1); the (reference,
+// axis, plane) triples of a round are numbered axis-major and dealt out one
+// per lane, each lane computing the triangle's bounds below and above its
+// plane (tri_split.h).  Bin b0 + i then gets the reference's box cut to "below
+// plane i" and "above plane i - 1" (the previous triple: the neighbouring lane,
+// or the last lane of the 32 before), bin b1 the box cut to "above plane m -
+// 1": sbvh.cu's binning, dealt out evenly.  A round is one warp's own: with
+// rounds of a whole block, their barriers were a fifth of the stalls.
+__device__ __forceinline__ void bin_spatial_rounds(const Pass& P, uint32_t p0, uint32_t p1, uint32_t stride,
+                                                   uint32_t* s_bin, const SpatialGrid& G, RoundTable& T) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (uint32_t r0 = p0; r0 < p1; r0 += stride) {
+        const bool here = r0 + lane < p1;
+        DBox mb;
+        box_reset(mb);
+        if (here) mb = ref_box(P.in[r0 + lane]);
+        uint32_t total = 0;
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {
+            uint32_t m = 0;
+            int b0 = 0;
+            const float scale = G.scale[k];
+            if (here && scale != 0.0f) m = bin_spatial_ends(s_bin, mb, k, G.lo[k], scale, &b0);
+            uint32_t x = m;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+                if (lane >= d) x += y;
+            }
+            T.cnt[32 * k + lane] = m;
+            T.off[32 * k + lane] = total + x - m;
+            T.b0[32 * k + lane] = (uint8_t)b0;
+            total += __shfl_sync(0xFFFFFFFFu, x, 31);
+        }
+        __syncwarp();
+        DBox carry;
+        box_reset(carry);
+#pragma unroll 1
+        for (uint32_t g0 = 0; g0 < total; g0 += 32) {
+            const uint32_t g = g0 + lane;
+            DBox below, above, rb;
+            box_reset(above);
+            int bin = -1, k = 0;
+            bool last = false;
+            uint32_t i = 0;
+            if (g < total) {
+                // the triple holding plane g: the last entry with off <= g (an
+                // entry without planes shares its offset with the next one, so
+                // that one has planes)
+                int a = 0, b = 3 * 32 - 1;
+                while (a < b) {
+                    const int mid = (a + b + 1) >> 1;
+                    if (T.off[mid] <= g) a = mid;
+                    else b = mid - 1;
+                }
+                k = a >> 5;
+                i = g - T.off[a];
+                last = i + 1 == T.cnt[a];
+                bin = T.b0[a] + (int)i;
+                const Ref r = P.in[r0 + (a & 31)];
+                rb = ref_box(r);
+                float tri[9];
+                load_tri(P.tris + 9 * (size_t)ref_prim(r), tri);
+                tri_plane_boxes(tri, k, plane_at(G.lo[k], G.hi[k], G.w[k], bin + 1), below, above);
+            }
+            DBox prev = shfl_up_box(above, 1);
+            if (lane == 0) prev = carry;
+            carry = shfl_box(above, 31);
+            if (g < total) bin_spatial_part(s_bin, k, bin, rb, i == 0, last, prev, below, above);
+        }
+        __syncwarp();  // the table is read
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_bin_spatial(Pass P) {
+    __shared__ uint32_t s_bin[3 * kBins * kSpWords];
+    __shared__ SpatialGrid s_grid;
+    __shared__ RoundTable s_table[kWarps];
+    __shared__ int s_last;
+    const uint32_t c = blockIdx.x;
+    BNode& N = P.nodes[P.chunk_node[c]];
+    if (!N.spatial) return;  // the whole block
+    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) init_bin_words(s_bin + kSpWords * i, kSpWords);
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        spatial_axis(N, k, &s_grid.lo[k], &s_grid.hi[k], &s_grid.w[k], &s_grid.scale[k]);
+    }
+    __syncthreads();
+    uint32_t p0, p1;
+    chunk_range(N, c, p0, p1);
+    const uint32_t warp = threadIdx.x >> 5;
+    bin_spatial_rounds(P, p0 + 32 * warp, p1, kThreads, s_bin, s_grid, s_table[warp]);
+    __syncthreads();
+    if (N.nchunks > 1 && !merge_bins(s_bin, P.bins + (size_t)N.bins * kBinWords + 3 * kBins * kObjWords, 3 * kBins,
+                                     kSpWords, &N.ctr[1], N.nchunks, &s_last))
+        return;
+    if (threadIdx.x >= 32) return;
+    int plane = 0;
+    const int sax = eval_spatial(s_bin, s_grid.scale, N.ocost, &plane);
+    if (threadIdx.x == 0 && sax >= 0) {
         N.kind = kSpatial;
         N.sax = sax;
-        N.splane = splane;
+        N.splane = plane_at(s_grid.lo[sax], s_grid.hi[sax], s_grid.w[sax], plane);
     }
 }
 
@@ -689,15 +753,15 @@ __device__ __forceinline__ void spatial_side(const Ref& r, const float* tris, in
                                              DBox& bl, DBox& br) {
     const DBox b = ref_box(r);
     bl = br = b;
-    if (b.hi[ax] <= pl) {
+    if (pick3(ax, b.hi[0], b.hi[1], b.hi[2]) <= pl) {
         to_l = true, to_r = false;
-    } else if (b.lo[ax] >= pl) {
+    } else if (pick3(ax, b.lo[0], b.lo[1], b.lo[2]) >= pl) {
         to_l = false, to_r = true;
     } else {
         float t[9];
         load_tri(tris + 9 * (size_t)ref_prim(r), t);
         DBox below, above;
-        tri_plane_bounds(t, ax, pl, below.lo, below.hi, above.lo, above.hi);
+        tri_plane_boxes(t, ax, pl, below, above);
         box_clip(bl, below);
         box_clip(br, above);
         to_l = !box_empty(bl);
@@ -743,7 +807,7 @@ __global__ void __launch_bounds__(kThreads) k_count(Pass P) {
             cnt[1] += rr;
         }
         if (op.axis >= 0) {
-            const bool l = bin_of(centroid(ref_box(r), op.axis), op.lo, op.scale) < op.plane;
+            const bool l = bin_of(centroid_at(ref_box(r), op.axis), op.lo, op.scale) < op.plane;
             cnt[2] += l;
             cnt[3] += !l;
         }
@@ -830,6 +894,10 @@ __global__ void __launch_bounds__(kThreads) k_count(Pass P) {
                 cf = atomicAdd(&P.ctr[kCtrSweep], 1u);
                 ok = ok && cf < P.cap_chunks;
                 s_sweep[s] = 1;
+            } else if (P.tris && m <= kSmallNode) {
+                cf = atomicAdd(&P.ctr[kCtrSmall], 1u);
+                ok = ok && cf < P.cap_chunks;
+                s_sweep[s] = 2;
             } else {
                 nchild = (m + kChunk - 1) / kChunk;
                 cf = atomicAdd(&P.ctr[kCtrChunks], nchild);
@@ -882,7 +950,7 @@ __global__ void __launch_bounds__(kThreads) k_count(Pass P) {
             C.spatial = 0;
             C.child[0] = C.child[1] = -1;
             C.leaf_cnt[0] = C.leaf_cnt[1] = 0;
-            if (s_sweep[s]) P.sweep_out[s_cf[s]] = (uint32_t)s_child[s];
+            if (s_sweep[s]) (s_sweep[s] == 1 ? P.sweep_out : P.small_out)[s_cf[s]] = (uint32_t)s_child[s];
         }
         for (uint32_t q = threadIdx.x; q < s_nch[s]; q += blockDim.x) P.chunk_out[s_cf[s] + q] = (uint32_t)s_child[s];
         if (s_slot[s] != 0xFFFFFFFFu) {
@@ -968,7 +1036,7 @@ __global__ void __launch_bounds__(kThreads) k_scatter(Pass P) {
                 spatial_side(r, P.tris, N.sax, N.splane, to[0], to[1], b[0], b[1]);
             } else {
                 b[0] = b[1] = ref_box(r);
-                const bool l = kind == kObject ? bin_of(centroid(b[0], op.axis), op.lo, op.scale) < op.plane
+                const bool l = kind == kObject ? bin_of(centroid_at(b[0], op.axis), op.lo, op.scale) < op.plane
                                                : (p - N.begin) < half;
                 to[0] = l;
                 to[1] = !l;
@@ -1023,6 +1091,199 @@ __global__ void __launch_bounds__(kThreads) k_scatter(Pass P) {
         dcen[s] = N.child[s] >= 0 ? P.nodes[N.child[s]].cb : nullptr;
     }
     reduce_side_boxes(acc, cen, s_red, dbox, dcen);
+}
+
+// ---------------------------------------------------------------------------
+// Small mesh-tree nodes: one warp each, all passes in one kernel
+// ---------------------------------------------------------------------------
+// The deep levels are hundreds of thousands of nodes of a few references,
+// where a block per node and pass left most lanes idle and wrote to memory
+// between passes what a warp keeps in registers: k_bin_object, k_bin_spatial,
+// k_count and k_scatter with the same decisions, two references a lane, the
+// bins in shared memory and the children's boxes by warp reductions.  The four
+// passes over the 1M-triangle scene took 40.5 ms (15.1 of them spatial binning);
+// they take 10.6 ms for the larger nodes and this kernel 12.9 ms (64 references
+// at most; at 32 it takes 8.8 ms, and the passes 4.9 ms more).
+constexpr int kSmallPer = (int)(kSmallNode / 32);
+struct SmallShared {
+    uint32_t bin[3 * kBins * kSpWords];
+    RoundTable table;
+    SpatialGrid grid;  // the axes' centroid grids, then the bin planes
+};
+
+__device__ __forceinline__ void reduce_box(const DBox& b, uint32_t* keys) {  // over the warp
+    for (int k = 0; k < 3; ++k) {
+        keys[k] = __reduce_min_sync(0xFFFFFFFFu, fkey(b.lo[k]));
+        keys[3 + k] = __reduce_max_sync(0xFFFFFFFFu, fkey(b.hi[k]));
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 5) k_small(Pass P, uint32_t count) {
+    __shared__ SmallShared s_all[kWarps];
+    const uint32_t item = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (item >= count) return;  // the whole warp
+    SmallShared& S = s_all[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    BNode& N = P.nodes[P.small_in[item]];
+    const uint32_t n = min(N.count, kSmallNode), begin = N.begin;
+    Ref r[kSmallPer];
+    bool have[kSmallPer];
+#pragma unroll
+    for (int q = 0; q < kSmallPer; ++q) {
+        have[q] = 32u * q + lane < n;
+        if (have[q]) r[q] = P.in[begin + 32 * q + lane];
+    }
+    // (loops that hold a reference split or a scan are not unrolled: with the
+    // code of both references and three axes side by side, fetching
+    // instructions was the first stall)
+    auto mine = [&](int q) { return q == 0 ? r[0] : r[kSmallPer - 1]; };
+    // ---- object split ----
+    if (lane < 3) object_axis(N, lane, &S.grid.lo[lane], &S.grid.scale[lane]);
+    for (int i = lane; i < 3 * kBins; i += 32) init_bin_words(S.bin + kObjWords * i, kObjWords);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kSmallPer; ++q)
+        if (have[q]) bin_object(S.bin, ref_box(r[q]), S.grid.lo, S.grid.scale);
+    __syncwarp();
+    const ObjectSplit o = eval_object(P, N, S.bin, S.grid.scale);
+    const float olo = o.axis >= 0 ? S.grid.lo[o.axis] : 0.0f, oscale = o.axis >= 0 ? S.grid.scale[o.axis] : 0.0f;
+    // ---- spatial split ----
+    int sax = -1;
+    float splane = 0.0f;
+    if (o.spatial) {
+        __syncwarp();
+        if (lane < 3) spatial_axis(N, lane, &S.grid.lo[lane], &S.grid.hi[lane], &S.grid.w[lane], &S.grid.scale[lane]);
+        for (int i = lane; i < 3 * kBins; i += 32) init_bin_words(S.bin + kSpWords * i, kSpWords);
+        __syncwarp();
+        bin_spatial_rounds(P, begin, begin + n, 32, S.bin, S.grid, S.table);
+        int plane = 0;
+        sax = eval_spatial(S.bin, S.grid.scale, o.cost, &plane);
+        if (sax >= 0) splane = plane_at(S.grid.lo[sax], S.grid.hi[sax], S.grid.w[sax], plane);
+    }
+    // ---- partition ----
+    bool to[kSmallPer][2];
+    DBox box[kSmallPer][2];
+    uint32_t mask[kSmallPer][2], total[2] = {0, 0};
+    auto ballots = [&]() {
+        total[0] = total[1] = 0;
+#pragma unroll
+        for (int q = 0; q < kSmallPer; ++q)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                mask[q][s] = __ballot_sync(0xFFFFFFFFu, to[q][s]);
+                total[s] += __popc(mask[q][s]);
+            }
+    };
+    bool spatial = sax >= 0;
+    if (spatial) {
+#pragma unroll 1
+        for (int q = 0; q < kSmallPer; ++q) {
+            bool l = false, rr = false;
+            DBox bl, br;
+            box_reset(bl);
+            box_reset(br);
+            if (32u * q + lane < n) spatial_side(mine(q), P.tris, sax, splane, l, rr, bl, br);
+#pragma unroll
+            for (int e = 0; e < kSmallPer; ++e)
+                if (e == q) {
+                    to[e][0] = l;
+                    to[e][1] = rr;
+                    box[e][0] = bl;
+                    box[e][1] = br;
+                }
+        }
+        ballots();
+        spatial = total[0] != 0 && total[1] != 0;  // an empty side: back to the object split
+    }
+    if (!spatial) {
+#pragma unroll
+        for (int q = 0; q < kSmallPer; ++q) {
+            to[q][0] = to[q][1] = false;
+            if (!have[q]) continue;
+            box[q][0] = box[q][1] = ref_box(r[q]);
+            const bool left = o.axis < 0 ? 32u * q + lane < n / 2
+                                         : bin_of(centroid_at(box[q][0], o.axis), olo, oscale) < o.plane;
+            to[q][0] = left;
+            to[q][1] = !left;
+        }
+        ballots();
+    }
+    // ---- children ----
+    int32_t child[2] = {-1, -1};
+    uint32_t first[2] = {0, 0}, slot[2] = {0, 0}, leaf[2] = {0, 0};
+    if (lane == 0) {
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t m = total[s];
+            if (m <= (uint32_t)P.leaf_max) {
+                first[s] = atomicAdd(&P.ctr[kCtrPool], m);
+                leaf[s] = first[s] + m <= P.cap_refs ? m : 0u;
+                if (leaf[s] != m) atomicExch(&P.ctr[kCtrOverflow], 1u);
+                if (leaf[s] != m) first[s] = 0;
+                continue;
+            }
+            const uint32_t nid = atomicAdd(&P.ctr[kCtrNodes], 1u);
+            first[s] = atomicAdd(&P.ctr[kCtrRefs], m);
+            slot[s] = atomicAdd(&P.ctr[kCtrSmall], 1u);
+            if (nid < P.cap_refs && first[s] + m <= P.cap_refs && slot[s] < P.cap_chunks) child[s] = (int32_t)nid;
+            else atomicExch(&P.ctr[kCtrOverflow], 1u);
+        }
+    }
+    for (int s = 0; s < 2; ++s) {
+        child[s] = __shfl_sync(0xFFFFFFFFu, child[s], 0);
+        first[s] = __shfl_sync(0xFFFFFFFFu, first[s], 0);
+        leaf[s] = __shfl_sync(0xFFFFFFFFu, leaf[s], 0);
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        DBox acc, cen;
+        box_reset(acc);
+        box_reset(cen);
+#pragma unroll
+        for (int q = 0; q < kSmallPer; ++q) {
+            if (!to[q][s]) continue;
+            uint32_t pos = __popc(mask[q][s] & lt);
+            for (int e = 0; e < q; ++e) pos += __popc(mask[e][s]);
+            const DBox& b = box[q][s];
+            box_grow(acc, b);
+            if (child[s] >= 0) {
+                P.out[first[s] + pos] = make_ref(b, ref_prim(r[q]));
+                for (int k = 0; k < 3; ++k) {
+                    const float ce = centroid(b, k);
+                    if (ce > -INFINITY && ce < INFINITY) {
+                        cen.lo[k] = fminf(cen.lo[k], ce);
+                        cen.hi[k] = fmaxf(cen.hi[k], ce);
+                    }
+                }
+            } else if (pos < leaf[s]) {
+                P.pool[first[s] + pos] = ref_prim(r[q]);
+            }
+        }
+        uint32_t bk[6], ck[6];
+        reduce_box(acc, bk);
+        reduce_box(cen, ck);
+        if (lane != 0) continue;
+        N.child[s] = child[s];
+        N.leaf_first[s] = first[s];
+        N.leaf_cnt[s] = leaf[s];
+        if (child[s] < 0) {
+            for (int k = 0; k < 6; ++k) N.lb[s][k] = bk[k];
+            continue;
+        }
+        BNode& C = P.nodes[child[s]];
+        for (int k = 0; k < 6; ++k) {
+            C.nb[k] = bk[k];
+            C.cb[k] = ck[k];
+            C.lb[0][k] = C.lb[1][k] = k < 3 ? kKeyPosInf : kKeyNegInf;
+        }
+        C.begin = first[s];
+        C.count = total[s];
+        C.set = N.set;
+        C.depth = N.depth + 1;
+        C.child[0] = C.child[1] = -1;
+        C.leaf_cnt[0] = C.leaf_cnt[1] = 0;
+        P.small_out[slot[s]] = (uint32_t)child[s];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1406,6 +1667,7 @@ __global__ void k_reset_level(uint32_t* ctr) {
     ctr[kCtrChunks] = 0;
     ctr[kCtrBins] = 0;
     ctr[kCtrSweep] = 0;
+    ctr[kCtrSmall] = 0;
 }
 
 __global__ void k_init_bins(uint32_t* bins, uint32_t slots) {
@@ -1532,6 +1794,8 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
     L_.bins1 = take(sizeof(uint32_t) * kBinWords * cap_bins);
     L_.sweep0 = take(sizeof(uint32_t) * cap_chunks);
     L_.sweep1 = take(sizeof(uint32_t) * cap_chunks);
+    L_.small0 = take(sizeof(uint32_t) * cap_chunks);
+    L_.small1 = take(sizeof(uint32_t) * cap_chunks);
     L_.ctr = take(sizeof(uint32_t) * kCtrs);
     L_.sets = take(sizeof(uint32_t) * 3 * std::max<uint32_t>(nsets, 1));  // root, offset, depth
     if (off > mem_bytes_) {
@@ -1546,12 +1810,13 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
     uint32_t* chunks[2] = {reinterpret_cast<uint32_t*>(m + L_.chunks0), reinterpret_cast<uint32_t*>(m + L_.chunks1)};
     uint32_t* bins[2] = {reinterpret_cast<uint32_t*>(m + L_.bins0), reinterpret_cast<uint32_t*>(m + L_.bins1)};
     uint32_t* sweeps[2] = {reinterpret_cast<uint32_t*>(m + L_.sweep0), reinterpret_cast<uint32_t*>(m + L_.sweep1)};
+    uint32_t* smalls[2] = {reinterpret_cast<uint32_t*>(m + L_.small0), reinterpret_cast<uint32_t*>(m + L_.small1)};
     uint32_t* ctr = reinterpret_cast<uint32_t*>(m + L_.ctr);
     uint32_t* sets = reinterpret_cast<uint32_t*>(m + L_.sets);
 
     // ---- level 0: a root per set of two or more primitives ----
     std::vector<BNode> roots;
-    std::vector<uint32_t> chunk_list, sweep_list;
+    std::vector<uint32_t> chunk_list, sweep_list, small_list;
     uint32_t nbins = 0;
     for (uint32_t s = 0; s < nsets; ++s) {
         const uint32_t n = counts[s];
@@ -1573,9 +1838,22 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         r.oax = r.sax = -1;
         r.child[0] = r.child[1] = -1;
         set_root_[s] = (uint32_t)roots.size();
+        if (triangles && n <= kSmallNode) {
+            small_list.push_back((uint32_t)roots.size());
+            r.chunk_first = 0;  // of the one chunk of its references' first pass
+            roots.push_back(r);
+            continue;
+        }
         for (uint32_t q = 0; q < r.nchunks; ++q) chunk_list.push_back((uint32_t)roots.size());
         if (n <= sweep_max) sweep_list.push_back((uint32_t)roots.size());
         roots.push_back(r);
+    }
+    // the first pass makes every root's references; the small roots' chunks
+    // come after the ones that the level passes take
+    uint32_t nchunks = sweep_list.empty() ? (uint32_t)chunk_list.size() : 0u;  // swept nodes are not binned
+    for (uint32_t id : small_list) {
+        roots[id].chunk_first = (uint32_t)chunk_list.size();
+        chunk_list.push_back(id);
     }
     if (roots.size() > cap || chunk_list.size() > cap_chunks || nbins > cap_bins) {
         *overflow = true;
@@ -1604,6 +1882,9 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         if (!sweep_list.empty())
             GB_CK(cudaMemcpyAsync(sweeps[0], sweep_list.data(), sizeof(uint32_t) * sweep_list.size(),
                                   cudaMemcpyHostToDevice, st));
+        if (!small_list.empty())
+            GB_CK(cudaMemcpyAsync(smalls[0], small_list.data(), sizeof(uint32_t) * small_list.size(),
+                                  cudaMemcpyHostToDevice, st));
         if (nbins) k_init_bins<<<div_up((size_t)nbins * 3 * kBins, 256), 256, 0, st>>>(bins[0], nbins);
         Pass P0{};
         P0.nodes = nodes;
@@ -1613,9 +1894,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         GB_CK(cudaGetLastError());
     }
     level_begin_.push_back((uint32_t)roots.size());
-    // chunks of nodes that are swept are not binned
-    uint32_t nchunks = sweep_list.empty() ? (uint32_t)chunk_list.size() : 0u;
-    uint32_t nsweep = (uint32_t)sweep_list.size();
+    uint32_t nsweep = (uint32_t)sweep_list.size(), nsmall = (uint32_t)small_list.size();
     uint32_t* host_ctr = nullptr;
     GB_CK(cudaMallocHost(&host_ctr, sizeof(uint32_t) * kCtrs));
     struct HostFree {
@@ -1623,7 +1902,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         ~HostFree() { cudaFreeHost(p); }
     } host_free{host_ctr};
     int cur = 0;
-    while (nchunks + nsweep > 0) {
+    while (nchunks + nsweep + nsmall > 0) {
         Pass P{};
         P.nodes = nodes;
         P.in = refs[cur];
@@ -1636,6 +1915,8 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         P.bins_out = bins[cur ^ 1];
         P.sweep_in = sweeps[cur];
         P.sweep_out = sweeps[cur ^ 1];
+        P.small_in = smalls[cur];
+        P.small_out = smalls[cur ^ 1];
         P.pool = reinterpret_cast<uint32_t*>(m + L_.pool);
         P.ctr = ctr;
         P.cap_refs = (uint32_t)std::min<size_t>(cap, 0xFFFFFFF0u);
@@ -1653,6 +1934,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
             k_count<<<nchunks, kThreads, 0, st>>>(P);
             k_scatter<<<nchunks, kThreads, 0, st>>>(P);
         }
+        if (nsmall) k_small<<<div_up(nsmall, kWarps), kThreads, 0, st>>>(P, nsmall);
         if (nsweep) {
             GB_CK(ensure_dynamic_smem(k_sweep, (int)kSweepSmem));
             k_sweep<<<nsweep, kSweepThreads, kSweepSmem, st>>>(P);
@@ -1667,6 +1949,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
         }
         nchunks = host_ctr[kCtrChunks];
         nsweep = host_ctr[kCtrSweep];
+        nsmall = host_ctr[kCtrSmall];
         level_begin_.push_back(host_ctr[kCtrNodes]);
         cur ^= 1;
         if (levels_ > 4096) return cudaErrorUnknown;  // cannot happen: every level splits nodes

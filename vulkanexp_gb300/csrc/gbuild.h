@@ -69,7 +69,7 @@ class GpuTreeBuilder {
     size_t mem_bytes_ = 0;
     struct Layout {
         size_t nodes, refs0, refs1, pool, chunks0, chunks1, chunk_cnt, chunk_off, bins0, bins1, ctr, sets, levels,
-            sweep0, sweep1;
+            sweep0, sweep1, small0, small1;
         size_t cap, cap_chunks, cap_bins;
     } L_{};
     std::vector<uint32_t> level_begin_;  // node ids of each level (levels + 1 entries)

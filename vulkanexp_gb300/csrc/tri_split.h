@@ -23,6 +23,8 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
+#include <string.h>
 
 #include "../../include/ddgi_exact.h"
 
@@ -56,59 +58,60 @@ DDGI_HD static inline float ts_div(float a, float b) {
     return a / b;
 #endif
 }
-// The neighbouring float above / below x.  Floats of one sign are ordered as
-// their bit patterns are, so on the device the neighbour is the pattern one
-// away (+0 stands for both zeros; +infinity and NaN stay): nextafterf's value
-// in six instructions.
+DDGI_HD static inline int32_t ts_bits(float x) {
+#ifdef __CUDA_ARCH__
+    return __float_as_int(x);
+#else
+    int32_t i;
+    memcpy(&i, &x, 4);
+    return i;
+#endif
+}
+DDGI_HD static inline float ts_float(int32_t i) {
+#ifdef __CUDA_ARCH__
+    return __int_as_float(i);
+#else
+    float x;
+    memcpy(&x, &i, 4);
+    return x;
+#endif
+}
+// The neighbouring float above / below x (nextafterf).  Floats of one sign are
+// ordered as their bit patterns are, so the neighbour is the pattern one away;
+// adding +0 makes one zero of the two, and +infinity is its own neighbour.
 DDGI_HD static inline float ts_up(float x) {
-#ifdef __CUDA_ARCH__
-    const int i = __float_as_int(__fadd_rn(x, 0.0f));
-    return x < INFINITY ? __int_as_float(i + ((i >> 31) | 1)) : x;
-#else
-    return nextafterf(x, INFINITY);
-#endif
+    const int32_t i = ts_bits(ts_add(x, 0.0f)), s = i >> 31, j = i + s + s + 1;
+    return ts_float(j < 0x7F800000 ? j : 0x7F800000);
 }
-DDGI_HD static inline float ts_down(float x) {
-#ifdef __CUDA_ARCH__
-    return -ts_up(-x);
-#else
-    return nextafterf(x, -INFINITY);
-#endif
-}
+DDGI_HD static inline float ts_down(float x) { return -ts_up(-x); }
 
 DDGI_HD static inline bool ts_crosses(float p, float q, float pl) { return (p < pl && q > pl) || (p > pl && q < pl); }
 
 // The crossing of edge p -> q with the plane x_K = pl, strictly between p and
-// q, added to the bounds of both sides.  t = (pl - p_K) / (q_K - p_K) lies in
-// (0, 1); numerator and denominator have the same sign, and rounding is
-// monotonic, so of the four quotients of their intervals' ends the lowest is
-// that of the smallest numerator and the largest denominator and the highest
-// the other way round (magnitudes), and of the four products of (q_a - p_a)
-// and t, t >= 0, the signs tell the lowest and the highest.
+// q: its bounds, added to lo/hi.  t = (pl - p_K) / (q_K - p_K) lies in (0, 1);
+// numerator and denominator have the same sign, and rounding is monotonic, so
+// of the four quotients of their intervals' ends the lowest is that of the
+// smallest numerator and the largest denominator (magnitudes) and the highest
+// the other way round, and of the four products of (q_a - p_a) and t, t >= 0,
+// the signs tell the lowest and the highest.
 template <int K>
-DDGI_HD static inline void ts_crossing(const float* p, const float* q, float pl, float llo[3], float lhi[3],
-                                       float glo[3], float ghi[3]) {
-    const float n = ts_sub(pl, p[K]), d = ts_sub(q[K], p[K]);
-    const float dlo = ts_down(d), dhi = ts_up(d);
+DDGI_HD static inline void ts_crossing(const float* p, const float* q, float pl, float lo[3], float hi[3]) {
+    // magnitudes: the interval's ends are the patterns one below and one above
+    const int32_t n = ts_bits(fabsf(ts_sub(pl, p[K]))), d = ts_bits(fabsf(ts_sub(q[K], p[K])));
     float t0 = 0.0f, t1 = 1.0f;
-    if (dlo > 0.0f || dhi < 0.0f) {
-        const float nlo = ts_down(n), nhi = ts_up(n);
-        const bool up = dlo > 0.0f;
-        t0 = fmaxf(0.0f, ts_down(ts_div(up ? nlo : nhi, up ? dhi : dlo)));
-        t1 = fminf(1.0f, ts_up(ts_div(up ? nhi : nlo, up ? dlo : dhi)));
+    if (d > 1) {
+        const float nhi = ts_float(n < 0x7F800000 ? n + 1 : n), dhi = ts_float(d < 0x7F800000 ? d + 1 : d);
+        const int32_t c0 = ts_bits(ts_div(ts_float(n - 1), dhi)) - 1;
+        t0 = ts_float(c0 > 0 ? c0 : 0);
+        t1 = fminf(1.0f, ts_up(ts_div(nhi, ts_float(d - 1))));
     }
+    lo[K] = hi[K] = pl;  // the crossing's own axis is the plane exactly
     for (int a = 0; a < 3; ++a) {
-        float clo = pl, chi = pl;  // the crossing's own axis is the plane exactly
-        if (a != K) {
-            const float dd = ts_sub(q[a], p[a]);
-            const float ddlo = ts_down(dd), ddhi = ts_up(dd);
-            clo = ts_down(ts_add(p[a], ts_down(ts_mul(ddlo, ddlo >= 0.0f ? t0 : t1))));
-            chi = ts_up(ts_add(p[a], ts_up(ts_mul(ddhi, ddhi >= 0.0f ? t1 : t0))));
-        }
-        llo[a] = fminf(llo[a], clo);
-        lhi[a] = fmaxf(lhi[a], chi);
-        glo[a] = fminf(glo[a], clo);
-        ghi[a] = fmaxf(ghi[a], chi);
+        if (a == K) continue;
+        const float dd = ts_sub(q[a], p[a]);
+        const float ddlo = ts_down(dd), ddhi = ts_up(dd);
+        lo[a] = fminf(lo[a], ts_down(ts_add(p[a], ts_down(ts_mul(ddlo, ddlo >= 0.0f ? t0 : t1)))));
+        hi[a] = fmaxf(hi[a], ts_up(ts_add(p[a], ts_up(ts_mul(ddhi, ddhi >= 0.0f ? t1 : t0)))));
     }
 }
 
@@ -147,8 +150,15 @@ DDGI_HD static inline void tri_plane_bounds_k(const float* tri, float pl, float 
         next[a] = v == 0 ? tri[3 + a] : (v == 1 ? tri[6 + a] : tri[a]);
         before[a] = v == 0 ? tri[6 + a] : (v == 1 ? tri[a] : tri[3 + a]);
     }
-    if (v == 0 ? c0 : (v == 1 ? c1 : c2)) ts_crossing<K>(at, next, pl, llo, lhi, glo, ghi);
-    if (v == 0 ? c2 : (v == 1 ? c0 : c1)) ts_crossing<K>(before, at, pl, llo, lhi, glo, ghi);
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (v == 0 ? c0 : (v == 1 ? c1 : c2)) ts_crossing<K>(at, next, pl, lo, hi);
+    if (v == 0 ? c2 : (v == 1 ? c0 : c1)) ts_crossing<K>(before, at, pl, lo, hi);
+    for (int a = 0; a < 3; ++a) {  // the crossings bound both sides
+        llo[a] = fminf(llo[a], lo[a]);
+        lhi[a] = fmaxf(lhi[a], hi[a]);
+        glo[a] = fminf(glo[a], lo[a]);
+        ghi[a] = fmaxf(ghi[a], hi[a]);
+    }
 }
 
 DDGI_HD static inline void tri_plane_bounds(const float* tri, int k, float pl, float llo[3], float lhi[3], float glo[3],
