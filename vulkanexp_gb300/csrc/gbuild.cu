@@ -1314,7 +1314,7 @@ __device__ void block_sort(unsigned long long* s_key, uint16_t* s_val, uint32_t 
 
 __device__ __forceinline__ float canon_zero(float x) { return x == 0.0f ? 0.0f : x; }
 
-// Inclusive block scan of boxes (kSweepPer consecutive elements per thread),
+// Inclusive block scan of boxes (up to kSweepPer consecutive elements per thread),
 // forward (prefix unions) or backward (suffix unions); out[i] gets the half
 // area of the union of elements [0, i] (forward) or [i, n) (backward).
 __device__ void box_scan_areas(const Ref* refs, const uint16_t* order, uint32_t n, bool forward, float* out,
@@ -1322,33 +1322,39 @@ __device__ void box_scan_areas(const Ref* refs, const uint16_t* order, uint32_t 
     const int t = threadIdx.x;
     DBox mine;
     box_reset(mine);
-    const int i0 = t * kSweepPer;
-    for (int e = 0; e < kSweepPer; ++e) {
+    const int per = (int)((n + kSweepThreads - 1) / kSweepThreads);  // at most kSweepPer
+    const int i0 = t * per;
+    for (int e = 0; e < per; ++e) {
         const int i = forward ? i0 + e : (int)n - 1 - (i0 + e);
         if (i < 0 || (uint32_t)i >= n) continue;
         box_grow(mine, ref_box(refs[order[i]]));
     }
-    for (int k = 0; k < 3; ++k) {
-        s_part[t][k] = mine.lo[k];
-        s_part[t][3 + k] = mine.hi[k];
+    // exclusive prefix over the threads: within the warp by shuffles, then the
+    // unions of the warps before (unions are exact in any order; one thread per
+    // component going through all 512 entries took most of a sweep)
+    const int lane = t & 31, warp = t >> 5;
+    DBox inc = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const DBox v = shfl_up_box(inc, o);
+        if (lane >= o) box_grow(inc, v);
     }
-    __syncthreads();
-    // exclusive prefix over threads (serial per component; 512 entries)
-    if (t < 6) {
-        float run = t < 3 ? INFINITY : -INFINITY;
-        for (int q = 0; q < kSweepThreads; ++q) {
-            const float v = s_part[q][t];
-            s_part[q][t] = run;
-            run = t < 3 ? fminf(run, v) : fmaxf(run, v);
+    if (lane == 31)
+        for (int k = 0; k < 3; ++k) {
+            s_part[warp][k] = inc.lo[k];
+            s_part[warp][3 + k] = inc.hi[k];
         }
-    }
     __syncthreads();
-    DBox acc;
-    for (int k = 0; k < 3; ++k) {
-        acc.lo[k] = s_part[t][k];
-        acc.hi[k] = s_part[t][3 + k];
+    DBox acc = shfl_up_box(inc, 1);
+    if (lane == 0) box_reset(acc);
+    for (int w = 0; w < warp; ++w) {
+        DBox v;
+        for (int k = 0; k < 3; ++k) {
+            v.lo[k] = s_part[w][k];
+            v.hi[k] = s_part[w][3 + k];
+        }
+        box_grow(acc, v);
     }
-    for (int e = 0; e < kSweepPer; ++e) {
+    for (int e = 0; e < per; ++e) {
         const int i = forward ? i0 + e : (int)n - 1 - (i0 + e);
         if (i < 0 || (uint32_t)i >= n) continue;
         box_grow(acc, ref_box(refs[order[i]]));
@@ -1358,9 +1364,9 @@ __device__ void box_scan_areas(const Ref* refs, const uint16_t* order, uint32_t 
 }
 
 // Dynamic shared memory of k_sweep: sort keys, prefix and suffix areas,
-// per-thread partial boxes, the sorted order of the current and best axis.
+// per-warp partial boxes, the sorted order of the current and best axis.
 constexpr size_t kSweepSmem = sizeof(unsigned long long) * kSweepMax + 2 * sizeof(float) * kSweepMax +
-                              sizeof(float) * 6 * kSweepThreads + 2 * sizeof(uint16_t) * kSweepMax;
+                              sizeof(float) * 6 * (kSweepThreads / 32) + 2 * sizeof(uint16_t) * kSweepMax;
 
 __global__ void __launch_bounds__(kSweepThreads) k_sweep(Pass P) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -1368,7 +1374,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_sweep(Pass P) {
     float* s_pre = reinterpret_cast<float*>(s_key + kSweepMax);
     float* s_suf = s_pre + kSweepMax;
     float(*s_part)[6] = reinterpret_cast<float(*)[6]>(s_suf + kSweepMax);
-    uint16_t* s_val = reinterpret_cast<uint16_t*>(s_suf + kSweepMax + 6 * kSweepThreads);
+    uint16_t* s_val = reinterpret_cast<uint16_t*>(s_suf + kSweepMax + 6 * (kSweepThreads / 32));
     uint16_t* s_best = s_val + kSweepMax;
     __shared__ float s_rc[kSweepThreads / 32];
     __shared__ uint32_t s_ro[kSweepThreads / 32], s_ri[kSweepThreads / 32];
@@ -1571,7 +1577,8 @@ __global__ void k_subtree(BNode* nodes, uint32_t b, uint32_t e, uint32_t* set_de
         N.dfs = 0;
         N.leaf_base = 0;
     }
-    atomicMax(set_depth + N.set, N.depth);
+    // (levels come deepest first: almost every node finds its set's depth there)
+    if (*(volatile const uint32_t*)(set_depth + N.set) < N.depth) atomicMax(set_depth + N.set, N.depth);
 }
 
 struct WriteArgs {
