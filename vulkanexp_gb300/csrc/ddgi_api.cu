@@ -879,12 +879,16 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
         (d->instance_count && !d->instances) || (d->offset_count && !d->offsets) ||
         (d->material_count && !d->materials))
         return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "null array with a non-zero count");
+    // object-space bounds of the meshes' triangles, taken on the way through
+    // their indices (a pass of its own took 16 ms for 3 M indices)
+    std::vector<float> mesh_lo((size_t)d->mesh_count * 3, INFINITY), mesh_hi((size_t)d->mesh_count * 3, -INFINITY);
     for (uint32_t m = 0; m < d->mesh_count; ++m) {
         const ddgi_mesh& me = d->meshes[m];
         if (me.index_count % 3) return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "mesh %u: index_count not a multiple of 3", m);
         if ((uint64_t)me.index_offset + me.index_count > d->index_count ||
             (uint64_t)me.vertex_offset + me.vertex_count > d->vertex_count)
             return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "mesh %u: range outside the vertex/index arrays", m);
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
         for (uint32_t i = 0; i < me.index_count; ++i) {
             const uint32_t v = d->indices[me.index_offset + i];
             if (v >= me.vertex_count)
@@ -892,7 +896,13 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
             const float* p = d->vertices[me.vertex_offset + v].pos;
             if (!std::isfinite(p[0]) || !std::isfinite(p[1]) || !std::isfinite(p[2]))
                 return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "mesh %u: vertex %u of a triangle is not finite", m, v);
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = p[k] < lo[k] ? p[k] : lo[k];
+                hi[k] = p[k] > hi[k] ? p[k] : hi[k];
+            }
         }
+        std::copy(lo, lo + 3, &mesh_lo[(size_t)m * 3]);
+        std::copy(hi, hi + 3, &mesh_hi[(size_t)m * 3]);
         if ((uint64_t)me.index_count / 3 >= (1ull << 28))
             return fail(ctx, DDGI_ERR_INVALID_ARGUMENT, "mesh %u: too many triangles", m);
     }
@@ -1060,7 +1070,6 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
     S.build_mode = ctx->build_mode;
     uint32_t host_blas_depth = 1;
     std::vector<int32_t> mesh_root(d->mesh_count, -1);
-    std::vector<float> mesh_lo((size_t)d->mesh_count * 3, INFINITY), mesh_hi((size_t)d->mesh_count * 3, -INFINITY);
     std::vector<int> gnode_base(d->mesh_count, 0), gprim_base(d->mesh_count, 0);
     std::vector<uint32_t> gorder_base(d->mesh_count, 0);
     uint64_t node_base = 0, tri_base = 0;
@@ -1068,16 +1077,6 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
         const ddgi_mesh& me = d->meshes[m];
         uint32_t nt = me.index_count / 3;
         if (nt == 0) continue;
-        for (uint32_t q = 0; q < me.index_count; ++q) {
-            const float4& p = pos[me.vertex_offset + d->indices[me.index_offset + q]];
-            float pp[3] = {p.x, p.y, p.z};
-            for (int k = 0; k < 3; ++k) {
-                if (pp[k] == pp[k]) {
-                    mesh_lo[m * 3 + k] = std::min(mesh_lo[m * 3 + k], pp[k]);
-                    mesh_hi[m * 3 + k] = std::max(mesh_hi[m * 3 + k], pp[k]);
-                }
-            }
-        }
         if (gpu_trees) {
             gnode_base[m] = (int)node_base;
             gprim_base[m] = (int)tri_base;

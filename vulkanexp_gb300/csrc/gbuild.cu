@@ -1902,12 +1902,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
     }
     level_begin_.push_back((uint32_t)roots.size());
     uint32_t nsweep = (uint32_t)sweep_list.size(), nsmall = (uint32_t)small_list.size();
-    uint32_t* host_ctr = nullptr;
-    GB_CK(cudaMallocHost(&host_ctr, sizeof(uint32_t) * kCtrs));
-    struct HostFree {
-        uint32_t* p;
-        ~HostFree() { cudaFreeHost(p); }
-    } host_free{host_ctr};
+    uint32_t host_ctr[kCtrs];  // (pinning memory for 32 bytes costs more than a build's copies)
     int cur = 0;
     while (nchunks + nsweep + nsmall > 0) {
         Pass P{};
@@ -1947,7 +1942,7 @@ cudaError_t GpuTreeBuilder::attempt(bool triangles, const float* tris, const flo
             k_sweep<<<nsweep, kSweepThreads, kSweepSmem, st>>>(P);
         }
         GB_CK(cudaGetLastError());
-        GB_CK(cudaMemcpyAsync(host_ctr, ctr, sizeof(uint32_t) * kCtrs, cudaMemcpyDeviceToHost, st));
+        GB_CK(cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, st));
         GB_CK(cudaStreamSynchronize(st));
         ++levels_;
         if (host_ctr[kCtrOverflow]) {
