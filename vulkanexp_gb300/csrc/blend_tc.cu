@@ -47,6 +47,8 @@ namespace ddgi {
 namespace {
 
 constexpr int kTileProbes = 25;    // 5 A rows per probe: (r, g, b, d, d^2); at most 25 (128 rows)
+constexpr int kMinTileProbes = 4;  // smallest tile of a launch that fills less than one round of CTAs
+constexpr int kMinRoundTile = 16;  // smallest tile of a launch of several rounds
 constexpr int kRowsPerProbe = 5;
 constexpr int kKChunk = 16;        // rays per shared-memory stage (one K step)
 constexpr int kStages = 4;         // operand stages in the ring
@@ -79,7 +81,8 @@ struct TcArgs {
     uint32_t* err;
     const uint32_t* dev_count;  // listed probes, read on the device (NULL: nprobes)
     uint32_t stall;             // test hook: issue no MMA and no commit, so the completion wait runs out
-    uint32_t tile;              // probes per CTA (1 .. kTileProbes)
+    uint32_t tile;              // probes per CTA (1 .. kTileProbes); with dev_count set on the device
+    uint32_t slots;             // CTAs resident at a time
     uint32_t smem_bytes;        // dynamic shared memory of the launch
     const float* hyst_dev;      // hysteresis of this update in device memory (the ramp's), or NULL: g.hyst
 };
@@ -623,8 +626,38 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
     }
 }
 
+// Probes per CTA for n probes where `slots` CTAs are resident at a time.
+// A CTA's time is a fixed part (the chunk pipeline, the accumulator
+// read-back) plus a part per probe.  Up to slots x kTileProbes probes one
+// round of CTAs takes them all, and the smallest tile that still fits in the
+// round is the fastest, down to kMinTileProbes, below which the fixed part
+// is all that is left (an update of 1,001 probes of 100 rays 176 -> 171 us, a
+// scheduled one of 333 of 2,048 probes 192 -> 185 us, against tiles of 16 and
+// more; a least tile of 2 or 8 is the same).  Beyond that the grid runs in rounds; the fixed part
+// is worth about 70 probes there (tiles of 25 / 20 / 18 / 16 probes over
+// 16,384 probes: 0.115 / 0.109 / 0.107 / 0.133 ms) and the size with the
+// fewest rounds x (70 + size) wins, the larger on ties.
+__host__ __device__ uint32_t tc_tile_size(uint32_t n, uint32_t slots) {
+    if (n <= slots * kTileProbes) {
+        const uint32_t t = (n + slots - 1) / slots;
+        return t < (uint32_t)kMinTileProbes ? (uint32_t)kMinTileProbes : t;
+    }
+    uint32_t best = kTileProbes, best_cost = ~0u;
+    for (uint32_t t = kTileProbes; t >= (uint32_t)kMinRoundTile; --t) {
+        const uint32_t rounds = ((n + t - 1) / t + slots - 1) / slots, cost = rounds * (70u + t);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = t;
+        }
+    }
+    return best;
+}
+
+// The tile follows the probes that are really listed: a scheduled update
+// knows that number on the device only.
 __global__ void __launch_bounds__(kThreads) k_blend_tc(TcArgs a) {
     const uint32_t n = a.dev_count ? *a.dev_count : a.nprobes;
+    if (a.dev_count) a.tile = tc_tile_size(n, a.slots);
     const uint32_t p0 = blockIdx.x * a.tile;
     if (p0 >= n) return;  // whole CTA, before any tensor-memory allocation
     blend_tc_tile(a, p0, n);
@@ -691,6 +724,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_blend_tc(BatchTables bt, Bat
         a.stall = 0;
         a.hyst_dev = nullptr;
         a.tile = kTileProbes;
+        a.slots = 0;
         a.smem_bytes = smem_bytes;
         s_v = v;
         s_tile = b - __ldg(bl.tile_base + lo);
@@ -703,34 +737,6 @@ __global__ void __launch_bounds__(kThreads) k_batch_blend_tc(BatchTables bt, Bat
         __threadfence();
         if (atomicAdd(bt.done + s_v, 1u) == s_items - 1u) bt.clock[1 + s_v] = globaltimer_ns();
     }
-}
-
-// Probes per CTA for a launch over n probes with `per_sm` CTAs resident per
-// SM: the grid runs in rounds of (SMs x per_sm) CTAs, and a CTA's time is
-// a fixed part (the chunk pipeline, the accumulator read-back) plus a part
-// per probe, measured on GB300 as about 70 probes' worth of fixed cost
-// (tiles of 25 / 20 / 18 / 16 probes over 16,384 probes: 0.115 / 0.109 /
-// 0.107 / 0.133 ms); the size with the fewest rounds x (70 + size) wins,
-// the larger on ties.
-uint32_t tc_tile_size(uint32_t n, uint32_t per_sm) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-                                                  cudaSuccess || sms <= 0) {
-        cudaGetLastError();
-        return kTileProbes;
-    }
-    const uint64_t slots = (uint64_t)sms * per_sm;
-    uint32_t best = kTileProbes;
-    uint64_t best_cost = ~0ull;
-    for (uint32_t t = kTileProbes; t >= 16; --t) {
-        const uint64_t tiles = (n + t - 1) / t, rounds = (tiles + slots - 1) / slots;
-        const uint64_t cost = rounds * (70 + t);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = t;
-        }
-    }
-    return best;
 }
 
 // Shared-memory limit of both blend kernels on the current device.
@@ -787,9 +793,15 @@ cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uin
     const size_t smem = tc_smem_bytes(nc, nd, Nc, Nd);
     cudaError_t e = set_tc_smem_limit();
     if (e != cudaSuccess) return e;
-    a.tile = tc_tile_size(nprobes, Nd + Nc > 256 ? 1u : 2u);
+    a.slots = (uint32_t)sm_count() * (Nd + Nc > 256 ? 1u : 2u);
+    a.tile = tc_tile_size(nprobes, a.slots);
     a.smem_bytes = (uint32_t)smem;
     uint32_t blocks = (nprobes + a.tile - 1) / a.tile;
+    if (dev_count) {  // any count up to nprobes: one round of the smallest tiles, or the several-round tiles
+        const uint32_t least = (nprobes + kMinTileProbes - 1) / kMinTileProbes;
+        const uint32_t most = (nprobes + kMinRoundTile - 1) / kMinRoundTile;
+        blocks = most > a.slots ? most : least < a.slots ? least : a.slots;
+    }
     k_blend_tc<<<blocks, kThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
