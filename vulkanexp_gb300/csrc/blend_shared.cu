@@ -73,7 +73,9 @@ __device__ __forceinline__ void texel_weights(const DeviceGrid& g, const float4*
 
 __global__ void __launch_bounds__(256) k_fp32_weights(DeviceGrid g, const float4* __restrict__ dirs, float* W,
                                                       float* wsum) {
+    let_next_launch();
     texel_weights(g, dirs, blockIdx.x * kWeightTexels, W, wsum);
+    after_previous();
 }
 
 // Words of a ray's records of TP probes in shared memory: r, g, b, depth of
@@ -89,25 +91,25 @@ __host__ __device__ constexpr uint32_t record_words() {
 // the next eight rays' weights are on their way while eight are used.
 // `step(w, row)` adds ray w's share.
 template <class Step>
-__device__ __forceinline__ void over_rays(const float* __restrict__ W, uint32_t ntex, uint32_t R, const float* rec,
+__device__ __forceinline__ void over_rays(const float* W, uint32_t ntex, uint32_t R, const float* rec,
                                           uint32_t words, Step step) {
     constexpr uint32_t U = 8;
     float w[U], next[U];
     const uint32_t full = R / U * U;
 #pragma unroll
-    for (uint32_t k = 0; k < U; ++k) next[k] = full ? __ldg(W + (size_t)k * ntex) : 0.0f;
+    for (uint32_t k = 0; k < U; ++k) next[k] = full ? W[(size_t)k * ntex] : 0.0f;
     for (uint32_t r = 0; r < full; r += U) {
 #pragma unroll
         for (uint32_t k = 0; k < U; ++k) w[k] = next[k];
         if (r + U < full) {
 #pragma unroll
-            for (uint32_t k = 0; k < U; ++k) next[k] = __ldg(W + (size_t)(r + U + k) * ntex);
+            for (uint32_t k = 0; k < U; ++k) next[k] = W[(size_t)(r + U + k) * ntex];
         }
 #pragma unroll
         for (uint32_t k = 0; k < U; ++k) step(pack2(w[k], w[k]), rec + (size_t)(r + k) * words);
     }
     for (uint32_t r = full; r < R; ++r) {
-        const float x = __ldg(W + (size_t)r * ntex);
+        const float x = W[(size_t)r * ntex];
         step(pack2(x, x), rec + (size_t)r * words);
     }
 }
@@ -296,6 +298,7 @@ __global__ void __launch_bounds__(kBlendThreads, 3) k_blend_fp32_shared(DeviceGr
                                                                         uint32_t* states, float4* color, float2* depth,
                                                                         const uint32_t* dev_count,
                                                                         const float* hyst_dev, uint32_t slots) {
+    after_previous();
     const uint32_t n = dev_count ? min(*dev_count, nprobes) : nprobes;
     const uint32_t tp = probes_per_block(n, slots);
     const float hy = hyst_dev ? *hyst_dev : g.hyst;
@@ -385,19 +388,23 @@ cudaError_t launch_color_weights(const DeviceGrid& g, const float4* dirs, float*
 cudaError_t launch_blend_fp32_shared(const DeviceGrid& g, const uint32_t* probe_list, uint32_t nprobes,
                                      const float4* rays, const float4* dirs, float* W, float* wsum, uint32_t* states,
                                      float4* color, float2* depth, cudaStream_t st, const uint32_t* dev_count,
-                                     const float* hyst_dev) {
+                                     const float* hyst_dev, bool early_weights) {
     if (nprobes == 0) return cudaSuccess;
     cudaError_t e = set_shared_smem_limit();
     if (e != cudaSuccess) return e;
     const uint32_t ntex = (g.color_res - 2) * (g.color_res - 2) + (g.depth_res - 2) * (g.depth_res - 2);
-    k_fp32_weights<<<weight_blocks(ntex), 256, weight_smem(g.rays), st>>>(g, dirs, W, wsum);
+    if (early_weights)
+        e = launch_dependent(k_fp32_weights, weight_blocks(ntex), 256, weight_smem(g.rays), st, g, dirs, W, wsum);
+    else
+        k_fp32_weights<<<weight_blocks(ntex), 256, weight_smem(g.rays), st>>>(g, dirs, W, wsum);
+    if (e != cudaSuccess) return e;
     const uint32_t slots = 3u * sm_count();
     // the most probes a block can be given decides its shared memory
     const size_t smem = nprobes >= 8u * slots ? blend_smem<8>(g.rays)
                                               : (nprobes >= 4u * slots ? blend_smem<4>(g.rays) : blend_smem<2>(g.rays));
-    k_blend_fp32_shared<<<min((nprobes + 1u) / 2u, slots), kBlendThreads, smem, st>>>(
-        g, probe_list, nprobes, rays, W, wsum, states, color, depth, dev_count, hyst_dev, slots);
-    return cudaGetLastError();
+    e = launch_dependent(k_blend_fp32_shared, min((nprobes + 1u) / 2u, slots), kBlendThreads, smem, st, g, probe_list,
+                         nprobes, rays, W, wsum, states, color, depth, dev_count, hyst_dev, slots);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_batch_blend_fp32_shared(const BatchTables& bt, const BatchBlendList& bl, uint32_t max_ntex,

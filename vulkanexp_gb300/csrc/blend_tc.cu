@@ -176,8 +176,10 @@ __device__ __forceinline__ void tc_weight_row(uint32_t row, uint32_t lane, const
 // One warp per row, four rows per block.
 __global__ void k_tc_weights(const float4* dirs, uint32_t R, uint32_t nc, uint32_t nd, float sharp, uint32_t Nc,
                              uint32_t Nd, uint32_t nchunks, uint8_t* wout, float* rowsum) {
+    let_next_launch();
     tc_weight_row(blockIdx.x * 4 + (threadIdx.x >> 5), threadIdx.x & 31, dirs, R, nc, nd, sharp, Nc, Nd, nchunks,
                   wout, rowsum);
+    after_previous();
 }
 
 // Calls put(bx, by) for each border texel of a tile of side n that copies
@@ -305,7 +307,7 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const uint32_t r = c * kKChunk + j * 2 + e;
-            v[e] = live && r < R ? __ldg(prec + r) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[e] = live && r < R ? prec[r] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
     load(va, 0);
@@ -656,6 +658,7 @@ __host__ __device__ uint32_t tc_tile_size(uint32_t n, uint32_t slots) {
 // The tile follows the probes that are really listed: a scheduled update
 // knows that number on the device only.
 __global__ void __launch_bounds__(kThreads) k_blend_tc(TcArgs a) {
+    after_previous();
     const uint32_t n = a.dev_count ? *a.dev_count : a.nprobes;
     if (a.dev_count) a.tile = tc_tile_size(n, a.slots);
     const uint32_t p0 = blockIdx.x * a.tile;
@@ -763,12 +766,19 @@ bool tc_blend_supported(uint32_t color_res, uint32_t depth_res) {
 cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uint32_t nprobes, const float4* rays,
                             const float4* dirs, uint8_t* wbuf, float* rowsum, uint32_t* states, void* color,
                             void* depth, float4* acc_color, float2* acc_depth, uint32_t* err, cudaStream_t st,
-                            const uint32_t* dev_count, bool stall, const float* hyst_dev) {
+                            const uint32_t* dev_count, bool stall, const float* hyst_dev, bool early_weights) {
     if (nprobes == 0) return cudaSuccess;
     const uint32_t nc = g.color_res - 2, nd = g.depth_res - 2;
     const uint32_t Nc = (nc * nc + 15) / 16 * 16, Nd = (nd * nd + 15) / 16 * 16;
     const uint32_t nchunks = (g.rays + kKChunk - 1) / kKChunk;
-    k_tc_weights<<<(Nd + Nc + 3) / 4, 128, 0, st>>>(dirs, g.rays, nc, nd, g.sharp, Nc, Nd, nchunks, wbuf, rowsum);
+    cudaError_t e = set_tc_smem_limit();
+    if (e != cudaSuccess) return e;
+    if (early_weights)
+        e = launch_dependent(k_tc_weights, (Nd + Nc + 3) / 4, 128, 0, st, dirs, g.rays, nc, nd, g.sharp, Nc, Nd,
+                             nchunks, wbuf, rowsum);
+    else
+        k_tc_weights<<<(Nd + Nc + 3) / 4, 128, 0, st>>>(dirs, g.rays, nc, nd, g.sharp, Nc, Nd, nchunks, wbuf, rowsum);
+    if (e != cudaSuccess) return e;
     TcArgs a;
     a.g = g;
     a.probe_list = probe_list;
@@ -791,8 +801,6 @@ cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uin
     a.stall = stall ? 1u : 0u;
     a.hyst_dev = hyst_dev;
     const size_t smem = tc_smem_bytes(nc, nd, Nc, Nd);
-    cudaError_t e = set_tc_smem_limit();
-    if (e != cudaSuccess) return e;
     a.slots = (uint32_t)sm_count() * (Nd + Nc > 256 ? 1u : 2u);
     a.tile = tc_tile_size(nprobes, a.slots);
     a.smem_bytes = (uint32_t)smem;
@@ -802,8 +810,8 @@ cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uin
         const uint32_t most = (nprobes + kMinRoundTile - 1) / kMinRoundTile;
         blocks = most > a.slots ? most : least < a.slots ? least : a.slots;
     }
-    k_blend_tc<<<blocks, kThreads, smem, st>>>(a);
-    return cudaGetLastError();
+    e = launch_dependent(k_blend_tc, blocks, kThreads, smem, st, a);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 uint32_t tc_tiles(uint32_t nprobes) { return (nprobes + kTileProbes - 1) / kTileProbes; }

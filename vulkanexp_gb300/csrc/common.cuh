@@ -30,6 +30,25 @@ __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t code) {
     if (err) atomicCAS(err, 0u, code);
 }
 
+// The kernels of an update follow one another on the stream, each reading what
+// the one before wrote.  Launched with launch_dependent, a kernel's blocks are
+// set up while the kernel before drains: it calls after_previous() before its
+// first use of anything that the kernels before it read or write, which
+// returns when they have finished and their writes can be seen (at once when
+// the kernel was launched in the ordinary way).  let_next_launch() allows the
+// next kernel's blocks to take the places that this one's leave.  A kernel
+// that runs ahead of its predecessor calls after_previous() as the last thing,
+// so that "finished" still means everything before it too.  What was written by
+// a kernel that can still be running is not read through the non-coherent path.
+// Of the wavefront update's kernels only the shadow rays and the weights let
+// the next launch begin early: with the closest-hit kernel doing so an update
+// of 16,384 probes took 6.84 ms instead of 6.47 (the next kernel's blocks wait
+// on its SMs), and in the shading kernels it changed nothing.  The launches
+// overlapped so, and the weights with the shadow rays' last blocks: 512 probes
+// of 128 rays 142 -> 128 us, 1,001 of 100 rays (BF16) 171 -> 156 us.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device wall clock in nanoseconds (for per-volume completion stamps).
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;

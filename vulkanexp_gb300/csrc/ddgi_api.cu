@@ -1379,17 +1379,20 @@ bool take_stall(ddgi_ctx* ctx) {
 // kernel that computes them per texel like the reference's shader (fused).
 // hyst: the ramp's hysteresis in device memory (NULL: the grid's); dcount:
 // the selected probe count on the device (NULL: n).
+// The weights may be computed while the kernel before still runs: the
+// directions were copied, and the weights last read, before the update's
+// first kernel.
 cudaError_t launch_blend(ddgi_ctx* ctx, const uint32_t* dlist, uint32_t n, cudaStream_t st,
                          const float* hyst = nullptr, const uint32_t* dcount = nullptr) {
     if (ctx->fp16)
         return launch_blend_tc(ctx->dg, dlist, n, ctx->rays, ctx->dirs, ctx->tc_weights, ctx->tc_rowsum, ctx->states,
                                ctx->color, ctx->depth, ctx->acc_color, ctx->acc_depth, ctx->err, st, dcount,
-                               take_stall(ctx), hyst);
+                               take_stall(ctx), hyst, true);
     if (ctx->pipeline == DDGI_PIPELINE_WAVEFRONT)
         return launch_blend_fp32_shared(ctx->dg, dlist, n, ctx->rays, ctx->dirs,
                                         reinterpret_cast<float*>(ctx->tc_weights), ctx->tc_rowsum, ctx->states,
                                         static_cast<float4*>(ctx->color), static_cast<float2*>(ctx->depth), st,
-                                        dcount, hyst);
+                                        dcount, hyst, true);
     return launch_blend_fp32(ctx->dg, dlist, n, ctx->rays, ctx->dirs, ctx->states, static_cast<float4*>(ctx->color),
                              static_cast<float2*>(ctx->depth), st, dcount, hyst);
 }

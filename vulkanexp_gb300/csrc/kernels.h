@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "common.cuh"
 
 namespace ddgi {
@@ -29,6 +31,24 @@ inline uint32_t sm_count() {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
         return 1u;
     return (uint32_t)sms;
+}
+
+// Launch of a kernel that calls after_previous() (common.cuh): its blocks may
+// be set up before the kernel that precedes it on the stream has finished.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t st,
+                                    A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // trace.cu
@@ -201,6 +221,9 @@ cudaError_t launch_adjoint_step(const DeviceScene& sc, const DeviceGrid& g, cons
                                 const float4* thit, const uint32_t* prim, const float4* gk, float4* gprev, float4* gx,
                                 float* W, float* wsum, double* grad, uint32_t* err, cudaStream_t st);
 
+// early_weights: nothing that is still running when the weights are launched
+// wrote `dirs` or reads the weights, so that they may be computed meanwhile.
+
 // blend_tc.cu
 size_t tc_weight_bytes(uint32_t rays, uint32_t color_res, uint32_t depth_res);
 bool tc_blend_supported(uint32_t color_res, uint32_t depth_res);
@@ -208,7 +231,7 @@ cudaError_t launch_blend_tc(const DeviceGrid& g, const uint32_t* probe_list, uin
                             const float4* dirs, uint8_t* wbuf, float* rowsum, uint32_t* states, void* color,
                             void* depth, float4* acc_color, float2* acc_depth, uint32_t* err, cudaStream_t st,
                             const uint32_t* dev_count = nullptr, bool stall = false,
-                            const float* hyst_dev = nullptr);
+                            const float* hyst_dev = nullptr, bool early_weights = false);
 
 // blend_shared.cu: FP32 blend with the weights computed once per update
 size_t fp32_weight_bytes(uint32_t rays, uint32_t color_res, uint32_t depth_res);
@@ -219,7 +242,7 @@ cudaError_t launch_color_weights(const DeviceGrid& g, const float4* dirs, float*
 cudaError_t launch_blend_fp32_shared(const DeviceGrid& g, const uint32_t* probe_list, uint32_t nprobes,
                                      const float4* rays, const float4* dirs, float* W, float* wsum, uint32_t* states,
                                      float4* color, float2* depth, cudaStream_t st, const uint32_t* dev_count = nullptr,
-                                     const float* hyst_dev = nullptr);
+                                     const float* hyst_dev = nullptr, bool early_weights = false);
 cudaError_t launch_batch_blend_fp32_shared(const BatchTables& bt, const BatchBlendList& bl, uint32_t max_ntex,
                                            uint32_t max_rays, const float4* rays, cudaStream_t st);
 

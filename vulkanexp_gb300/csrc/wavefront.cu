@@ -188,6 +188,8 @@ template <class Stack, template <bool, class> class Walker>
 __global__ void __launch_bounds__(kPersistThreads, Walker<false, Stack>::kMinBlocks) k_shadow(DeviceScene sc, ShadowJob job, const uint32_t* qcount,
                                                                uint32_t* counter, int stack_cap, int split, WalkKnobs knobs,
                                                                uint32_t* err) {
+    after_previous();
+    let_next_launch();  // the blend weights start in the places that the last rays leave
     persistent_walk<true, Stack, Walker>(sc, job, *qcount, counter, stack_cap, split, knobs, err);
 }
 
@@ -209,6 +211,7 @@ __device__ __forceinline__ uint32_t warp_append(bool flag, uint32_t* count) {
 __global__ void __launch_bounds__(128) k_shade_classify(DeviceGrid g, DeviceLight L, uint32_t total, WaveHits hits,
                                                         float4* rays_out, ddgi_hit* hits_out, uint32_t* front_count,
                                                         const uint32_t* dev_count) {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (dev_count) total = *dev_count * g.rays;
     bool is_front = false;
@@ -246,6 +249,7 @@ __global__ void __launch_bounds__(128, 5) k_shade_front(DeviceScene sc, DeviceGr
                                                         const uint32_t* __restrict__ states, AV at, WaveHits hits,
                                                         const uint32_t* front_count, float4* rays_out, ShadowQueue q,
                                                         uint32_t* err) {
+    after_previous();
     const uint32_t n = *front_count;
     if (blockIdx.x * blockDim.x >= n) return;  // whole block
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -523,23 +527,26 @@ cudaError_t wavefront_kernels(const DeviceScene& sc, const DeviceGrid& g, const 
     ShadowQueue qq = q;
     qq.count = counters + 1;
     uint32_t blocks = (total + 127) / 128;
-    k_shade_classify<<<blocks, 128, 0, st>>>(g, L, total, hits, rays_out, hits_out, counters + 3, dev_count);
+    cudaError_t e = launch_dependent(k_shade_classify, blocks, 128, 0, st, g, L, total, hits, rays_out, hits_out,
+                                     counters + 3, dev_count);
+    if (e != cudaSuccess) return e;
     if (fp16_atlas) {
         AtlasView<ColorTexF16, DepthTexF16> at{{static_cast<const uint2*>(color)},
                                                {static_cast<const uint32_t*>(depth)}};
-        k_shade_front<<<blocks, 128, 0, st>>>(sc, g, L, probe_list, dirs, states, at, hits, counters + 3, rays_out, qq,
-                                              err);
+        e = launch_dependent(k_shade_front<decltype(at)>, blocks, 128, 0, st, sc, g, L, probe_list, dirs, states, at,
+                             hits, counters + 3, rays_out, qq, err);
     } else {
         AtlasView<ColorTexF32, DepthTexF32> at{{static_cast<const float4*>(color)},
                                                {static_cast<const float2*>(depth)}};
-        k_shade_front<<<blocks, 128, 0, st>>>(sc, g, L, probe_list, dirs, states, at, hits, counters + 3, rays_out, qq,
-                                              err);
+        e = launch_dependent(k_shade_front<decltype(at)>, blocks, 128, 0, st, sc, g, L, probe_list, dirs, states, at,
+                             hits, counters + 3, rays_out, qq, err);
     }
+    if (e != cudaSuccess) return e;
     ShadowJob sj{qq, make_float3(L.dir[0], L.dir[1], L.dir[2]), rays_out, hits.prim, 0};
-    k_shadow<Stack, Walker><<<persistent_blocks((const void*)k_shadow<Stack, Walker>, smem, tune.ctas_per_sm),
-                              kPersistThreads, smem, st>>>(sc, sj, counters + 1, counters + 2, stack_cap, split, knobs,
-                                                           err);
-    return cudaGetLastError();
+    e = launch_dependent(k_shadow<Stack, Walker>,
+                         persistent_blocks((const void*)k_shadow<Stack, Walker>, smem, tune.ctas_per_sm),
+                         kPersistThreads, smem, st, sc, sj, counters + 1, counters + 2, stack_cap, split, knobs, err);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace
