@@ -3,6 +3,8 @@ blend weights with the shadow rays: updates queued one after another (a new
 direction table each, so that weights computed too early would show) must
 equal updates with the stream drained in between, bit for bit, and so must an
 update captured in a graph and replayed."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -31,6 +33,7 @@ def run(precision, scheduled, mode):
     st.synchronize()
     if mode == "captured":
         graph = torch.cuda.CUDAGraph()
+        gc.collect()  # a context collected during the capture would free device memory, which a capture forbids
         with torch.cuda.graph(graph, stream=st, capture_error_mode="thread_local"):
             update(1)
         with torch.cuda.stream(st):

@@ -1518,23 +1518,24 @@ ddgi_status ddgi_update_scheduled(ddgi_ctx* ctx, const float orientation[9], uin
     ddgi_status s = prepare_update(ctx, orientation, nullptr, 0, st, &unused, &P);
     if (s != DDGI_OK) return s;
     uint32_t* dcount = ctx->sched + 2;
+    const uint32_t most = max_probes != 0 && max_probes < P ? max_probes : P;  // that *dcount can be
     if (ctx->timing) CK(cudaEventRecord(ctx->ev[0], st), "event");
     CK(launch_select_probes(ctx->states, P, max_probes, ctx->sched, ctx->probe_list, st), "schedule launch");
     WaveHits wh{ctx->wave_thit, ctx->wave_prim, ctx->wave_front};
     ShadowQueue q{ctx->q_idx, ctx->q_pos, ctx->q_sun, nullptr};
     ddgi_hit* hits_out = ctx->record_hits ? ctx->hits : nullptr;
-    CK(launch_wavefront(device_scene(ctx), ctx->dg, ctx->dl, ctx->probe_list, P, ctx->dirs, ctx->ray_order,
+    CK(launch_wavefront(device_scene(ctx), ctx->dg, ctx->dl, ctx->probe_list, most, ctx->dirs, ctx->ray_order,
                         ctx->states, ctx->color, ctx->depth, ctx->fp16, wh, q, ctx->counters, ctx->rays, hits_out,
                         ctx->scene.stack_cap, ctx->scene.wstack_cap, ctx->err, st,
                         ctx->timing ? ctx->ev[3] : nullptr, dcount, trace_tuning(ctx), nullptr),
        "wavefront trace launch");
     if (ctx->dl.sky_mode == DDGI_SKY_ATMOSPHERE)
-        CK(launch_shade_sky(ctx->dg, ctx->dl, P, dcount, ctx->probe_list, ctx->dirs, ctx->rays, st), "sky launch");
+        CK(launch_shade_sky(ctx->dg, ctx->dl, most, dcount, ctx->probe_list, ctx->dirs, ctx->rays, st), "sky launch");
     if (ctx->timing) CK(cudaEventRecord(ctx->ev[1], st), "event");
     cudaError_t re;
     const float* hyst = ramp_step(ctx, dcount, 0, st, &re);
     CK(re, "hysteresis ramp launch");
-    CK(launch_blend(ctx, ctx->probe_list, P, st, hyst, dcount), "blend launch");
+    CK(launch_blend(ctx, ctx->probe_list, most, st, hyst, dcount), "blend launch");
     if (ctx->timing) {
         CK(cudaEventRecord(ctx->ev[2], st), "event");
         ctx->timing_pending = true;

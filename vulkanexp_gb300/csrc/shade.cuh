@@ -90,6 +90,16 @@ __device__ __forceinline__ float3 grid_probe_pos(const DeviceGrid& g, int x, int
 __device__ __forceinline__ float dot_fma(float3 a, float3 b) {
     return fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x)));
 }
+// The products and sums of a hit's surface and of its sun term, each rounded in
+// one way in every kernel that shades hits.
+__device__ __forceinline__ float mix_of_three(float x, float a, float y, float b, float z, float c) {
+    return fmaf(z, c, fmaf(x, a, __fmul_rn(y, b)));
+}
+__device__ __forceinline__ float dot_hit(float3 a, float3 b) { return mix_of_three(a.x, b.x, a.y, b.y, a.z, b.z); }
+__device__ __forceinline__ float3 norm_hit(float3 a) {
+    const float k = 1.0f / sqrtf(dot_hit(a, a));
+    return f3(__fmul_rn(a.x, k), __fmul_rn(a.y, k), __fmul_rn(a.z, k));
+}
 __device__ __forceinline__ float sqrt_approx(float v) {  // within 2^-23 relative (PTX sqrt.approx)
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -240,6 +250,65 @@ __device__ __forceinline__ void probe_weights(const CellProbe& p, float3 bv, flo
     *weight = __fmul_rn(w, p.triw);
 }
 
+// The biased position itself is rounded, as in the reference: where the
+// distance from it is the stored mean distance, visibility jumps.
+__device__ __forceinline__ float3 biased_position(float3 position, float3 normal, float3 toCamera,
+                                                  const DeviceGrid& g) {
+    return f3(fmaf(normal.x + toCamera.x, g.bias, position.x), fmaf(normal.y + toCamera.y, g.bias, position.y),
+              fmaf(normal.z + toCamera.z, g.bias, position.z));
+}
+
+// What probe p gives to one lookup: its irradiance's square root, its weight
+// and its weight without visibility.
+struct ProbeShare {
+    float r[3];
+    float weight, fallback;
+};
+template <class AV>
+__device__ __forceinline__ ProbeShare probe_share(const CellProbe& p, float3 biasedPosition, float3 normal, float2 nuv,
+                                                  const LookupScales& s, const DeviceGrid& g, const AV& at) {
+    const Tap t = atlas_tap(p.tile + s.cinv, p.z + s.cinv, nuv, s.cscale, s.cr, g.color_w, g.color_h);
+    float c00[3], c10[3], c01[3], c11[3];
+    at.color.fetch(t.row0, c00);
+    at.color.fetch(t.row0 + 1u, c10);
+    at.color.fetch(t.row1, c01);
+    at.color.fetch(t.row1 + 1u, c11);
+    ProbeShare x;
+    probe_weights(p, p.at - biasedPosition, normal, at.depth, s, g, &x.weight, &x.fallback);
+    const float w11 = __fmul_rn(t.ax, t.ay), w10 = t.ax - w11, w01 = t.ay - w11, w00 = 1.0f - t.ax - w01;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        x.r[k] = sqrt_approx(fmaf(w11, c11[k], fmaf(w01, c01[k], fmaf(w10, c10[k], __fmul_rn(w00, c00[k])))));
+    return x;
+}
+
+// The probes' shares of one lookup added up in their order.
+struct LookupSum {
+    float final[3] = {0.0f, 0.0f, 0.0f}, other[3] = {0.0f, 0.0f, 0.0f};
+    float weight = 0.0f, fallback = 0.0f;
+
+    __device__ __forceinline__ void add(const ProbeShare& x) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) final[k] = fmaf(x.r[k], x.weight, final[k]);
+        weight += x.weight;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) other[k] = fmaf(x.r[k], x.fallback, other[k]);
+        fallback += x.fallback;
+    }
+    __device__ __forceinline__ float3 color() const {
+        const float n = weight > 1e-3f ? 1.0f / weight : 1.0f;
+        const float nf = fallback > 1e-3f ? 1.0f / fallback : 1.0f;
+        const float k = 8.0f * clampf(weight, 0.0f, 1.0f / 8.0f);
+        float r[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float fc = __fmul_rn(final[c], n), fb = __fmul_rn(other[c], nf);
+            r[c] = fmaf(__fmul_rn(fb, fb), 1.0f - k, __fmul_rn(__fmul_rn(fc, fc), k));
+        }
+        return f3(r[0], r[1], r[2]);
+    }
+};
+
 // sampleProbes (src/shaders/irradiance.glsl:145-237) for NQ lookups at one
 // position that differ in the direction argument (`normal`): the closest-hit
 // program makes two (reflection and diffuse), which share the eight probes'
@@ -265,61 +334,55 @@ __device__ void sample_probes_n(float3 position, const float3 (&normal)[NQ], flo
     const LookupScales s = lookup_scales(g);
     float3 biasedPosition[NQ];
     float2 nuv[NQ];
-    float3 finalColor[NQ], fallbackColor[NQ];
-    float totalWeight[NQ], totalFallbackWeight[NQ];
+    LookupSum sum[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
-        // the biased position itself is rounded, as in the reference: where
-        // the distance from it is the stored mean distance, visibility jumps
-        biasedPosition[q] = f3(fmaf(normal[q].x + toCamera.x, g.bias, position.x),
-                               fmaf(normal[q].y + toCamera.y, g.bias, position.y),
-                               fmaf(normal[q].z + toCamera.z, g.bias, position.z));
+        biasedPosition[q] = biased_position(position, normal[q], toCamera, g);
         nuv[q] = oct_uv(normal[q]);
-        finalColor[q] = fallbackColor[q] = f3(0, 0, 0);
-        totalWeight[q] = totalFallbackWeight[q] = 0.0f;
     }
 #pragma unroll 1
     for (uint32_t live = cell.live; live != 0u; live &= live - 1u) {
         const CellProbe p = cell_probe(cell, (uint32_t)__ffs((int)live) - 1u, position, g);
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const Tap t = atlas_tap(p.tile + s.cinv, p.z + s.cinv, nuv[q], s.cscale, s.cr, g.color_w, g.color_h);
-            float c00[3], c10[3], c01[3], c11[3];
-            at.color.fetch(t.row0, c00);
-            at.color.fetch(t.row0 + 1u, c10);
-            at.color.fetch(t.row1, c01);
-            at.color.fetch(t.row1 + 1u, c11);
-            float weight, fallbackWeight;
-            probe_weights(p, p.at - biasedPosition[q], normal[q], at.depth, s, g, &weight, &fallbackWeight);
-            const float w11 = __fmul_rn(t.ax, t.ay), w10 = t.ax - w11, w01 = t.ay - w11, w00 = 1.0f - t.ax - w01;
-            float r[3];
+        for (int q = 0; q < NQ; ++q)
+            sum[q].add(probe_share(p, biasedPosition[q], normal[q], nuv[q], s, g, at));
+    }
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
-                r[k] = sqrt_approx(fmaf(w11, c11[k], fmaf(w01, c01[k], fmaf(w10, c10[k], __fmul_rn(w00, c00[k])))));
-            finalColor[q] = f3(fmaf(r[0], weight, finalColor[q].x), fmaf(r[1], weight, finalColor[q].y),
-                               fmaf(r[2], weight, finalColor[q].z));
-            totalWeight[q] += weight;
-            fallbackColor[q] = f3(fmaf(r[0], fallbackWeight, fallbackColor[q].x),
-                                  fmaf(r[1], fallbackWeight, fallbackColor[q].y),
-                                  fmaf(r[2], fallbackWeight, fallbackColor[q].z));
-            totalFallbackWeight[q] += fallbackWeight;
+    for (int q = 0; q < NQ; ++q) result[q] = sum[q].color();
+}
+
+// One lookup by PARTS neighbouring lanes of a warp, all of which call it (those
+// without a lookup with `valid` false): each takes every PARTS-th of the eight
+// probes, and all add the shares up in the probes' order, so that the sums are
+// sample_probes_n's bit for bit.
+template <int PARTS, class AV>
+__device__ __forceinline__ float3 sample_probes_split(bool valid, float3 position, float3 normal, float3 toCamera,
+                                                      const DeviceGrid& g, const uint32_t* states, const AV& at) {
+    ProbeCell cell;
+    if (!valid || !probe_cell(position, g, states, &cell)) cell.live = 0u;
+    const uint32_t lane = threadIdx.x & 31u, part = lane % PARTS, lead = lane - part;
+    const LookupScales s = lookup_scales(g);
+    const float3 biased = biased_position(position, normal, toCamera, g);
+    const float2 nuv = oct_uv(normal);
+    LookupSum sum;
+#pragma unroll 1
+    for (uint32_t j = 0; j < 8u; j += PARTS) {
+        ProbeShare own = {{0.0f, 0.0f, 0.0f}, 0.0f, 0.0f};  // a share of nothing changes no sum
+        if (cell.live >> (j + part) & 1u)
+            own = probe_share(cell_probe(cell, j + part, position, g), biased, normal, nuv, s, g, at);
+#pragma unroll
+        for (uint32_t p = 0; p < (uint32_t)PARTS; ++p) {
+            ProbeShare x = own;
+            if (PARTS > 1) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) x.r[k] = __shfl_sync(0xffffffffu, own.r[k], lead + p);
+                x.weight = __shfl_sync(0xffffffffu, own.weight, lead + p);
+                x.fallback = __shfl_sync(0xffffffffu, own.fallback, lead + p);
+            }
+            sum.add(x);
         }
     }
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const float n = totalWeight[q] > 1e-3f ? 1.0f / totalWeight[q] : 1.0f;
-        const float nf = totalFallbackWeight[q] > 1e-3f ? 1.0f / totalFallbackWeight[q] : 1.0f;
-        const float k = 8.0f * clampf(totalWeight[q], 0.0f, 1.0f / 8.0f);
-        const float fc[3] = {__fmul_rn(finalColor[q].x, n), __fmul_rn(finalColor[q].y, n),
-                             __fmul_rn(finalColor[q].z, n)};
-        const float fb[3] = {__fmul_rn(fallbackColor[q].x, nf), __fmul_rn(fallbackColor[q].y, nf),
-                             __fmul_rn(fallbackColor[q].z, nf)};
-        float r[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            r[c] = fmaf(__fmul_rn(fb[c], fb[c]), 1.0f - k, __fmul_rn(__fmul_rn(fc[c], fc[c]), k));
-        result[q] = f3(r[0], r[1], r[2]);
-    }
+    return sum.color();
 }
 
 template <class AV>
@@ -335,33 +398,40 @@ __device__ __forceinline__ float3 sample_probes(float3 position, float3 normal, 
 __device__ __forceinline__ float3 pbr_metallic_roughness(float3 n, float3 v, float3 lightColor, float3 lightDir,
                                                          float3 albedo, float metal, float rough) {
     const float pi = DDGI_PI;
-    float3 diffuseColor = albedo * (1.0f - 0.04f) * (1.0f - metal);
-    float alphaRoughness = rough * rough;
-    float3 specularColor = mix3(f3(0.04f, 0.04f, 0.04f), albedo, metal);
-    float reflectance = fmaxf(fmaxf(specularColor.x, specularColor.y), specularColor.z);
-    float reflectance90 = clampf(reflectance * 25.0f, 0.0f, 1.0f);
-    float3 R0 = specularColor;
-    float3 R90 = f3(reflectance90, reflectance90, reflectance90);
-    float3 l = norm3(lightDir);
-    float3 h = norm3(l + v);
-    float NdotL = clampf(dot3(n, l), 0.001f, 1.0f);
-    float NdotV = clampf(fabsf(dot3(n, v)), 0.001f, 1.0f);
-    float NdotH = clampf(dot3(n, h), 0.0f, 1.0f);
-    float VdotH = clampf(dot3(v, h), 0.0f, 1.0f);
-    float x = clampf(1.0f - VdotH, 0.0f, 1.0f);
-    float x2 = x * x;
-    float p5 = x2 * x2 * x;
-    float3 F = R0 + (R90 - R0) * p5;
-    float a2 = alphaRoughness * alphaRoughness;
-    float attL = 2.0f * NdotL / (NdotL + sqrtf(a2 + (1.0f - a2) * (NdotL * NdotL)));
-    float attV = 2.0f * NdotV / (NdotV + sqrtf(a2 + (1.0f - a2) * (NdotV * NdotV)));
-    float G = attL * attV;
-    float a = NdotH * alphaRoughness;
-    float k = alphaRoughness / ((1.0f - NdotH * NdotH) + a * a);
-    float D = clampf(k * k * (1.0f / pi), 0.0f, 4.0f);
-    float3 diffuseContrib = (f3(1, 1, 1) - F) * diffuseColor * (1.0f / pi);
-    float3 specContrib = F * (G * D / (4.0f * NdotL * NdotV));
-    return lightColor * (diffuseContrib + specContrib) * NdotL;
+    const float alphaRoughness = __fmul_rn(rough, rough), dull = 1.0f - metal;
+    const float al[3] = {albedo.x, albedo.y, albedo.z}, lc[3] = {lightColor.x, lightColor.y, lightColor.z};
+    float R0[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) R0[c] = fmaf(0.04f, dull, __fmul_rn(al[c], metal));
+    const float reflectance = fmaxf(fmaxf(R0[0], R0[1]), R0[2]);
+    const float R90 = clampf(__fmul_rn(reflectance, 25.0f), 0.0f, 1.0f);
+    const float3 l = norm_hit(lightDir);
+    const float3 h = norm_hit(l + v);
+    const float NdotL = clampf(dot_hit(n, l), 0.001f, 1.0f);
+    const float NdotV = clampf(fabsf(dot_hit(n, v)), 0.001f, 1.0f);
+    const float NdotH = clampf(dot_hit(n, h), 0.0f, 1.0f);
+    const float VdotH = clampf(dot_hit(v, h), 0.0f, 1.0f);
+    const float x = clampf(1.0f - VdotH, 0.0f, 1.0f);
+    const float x2 = __fmul_rn(x, x);
+    const float p5 = __fmul_rn(__fmul_rn(x2, x2), x);
+    const float rest = fmaf(-alphaRoughness, alphaRoughness, 1.0f);
+    const float attL = __fmul_rn(2.0f, NdotL) /
+                       (NdotL + sqrtf(fmaf(alphaRoughness, alphaRoughness, __fmul_rn(rest, __fmul_rn(NdotL, NdotL)))));
+    const float attV = __fmul_rn(2.0f, NdotV) /
+                       (NdotV + sqrtf(fmaf(alphaRoughness, alphaRoughness, __fmul_rn(rest, __fmul_rn(NdotV, NdotV)))));
+    const float a = __fmul_rn(NdotH, alphaRoughness);
+    const float k = alphaRoughness / fmaf(a, a, fmaf(-NdotH, NdotH, 1.0f));
+    const float D = clampf(__fmul_rn(__fmul_rn(k, k), 1.0f / pi), 0.0f, 4.0f);
+    const float spec = __fmul_rn(__fmul_rn(attL, attV), D) / __fmul_rn(__fmul_rn(4.0f, NdotL), NdotV);
+    float out[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float F = fmaf(R90 - R0[c], p5, R0[c]);
+        const float diffuse = __fmul_rn(__fmul_rn(al[c], 1.0f - 0.04f), dull);
+        const float both = fmaf(__fmul_rn(1.0f - F, diffuse), 1.0f / pi, __fmul_rn(F, spec));
+        out[c] = __fmul_rn(__fmul_rn(lc[c], both), NdotL);
+    }
+    return f3(out[0], out[1], out[2]);
 }
 
 // Front-face hit shading of src/shaders/closesthit.glsl:143-286 (NO_REFLECTION,
@@ -400,12 +470,13 @@ __device__ __forceinline__ bool surface_at(const DeviceScene& sc, float3 origin,
     }
     float4 n0 = __ldg(sc.normals + vb + i0), n1 = __ldg(sc.normals + vb + i1), n2 = __ldg(sc.normals + vb + i2);
     float b0 = 1.0f - b1 - b2;
-    float3 tsn = norm3(f3(n0.x * b0 + n1.x * b1 + n2.x * b2, n0.y * b0 + n1.y * b1 + n2.y * b2,
-                          n0.z * b0 + n1.z * b1 + n2.z * b2));
+    float3 tsn = norm_hit(f3(mix_of_three(n0.x, b0, n1.x, b1, n2.x, b2), mix_of_three(n0.y, b0, n1.y, b1, n2.y, b2),
+                             mix_of_three(n0.z, b0, n1.z, b1, n2.z, b2)));
     float4 w0 = __ldg(&gi->w2o[0]), w1 = __ldg(&gi->w2o[1]), w2 = __ldg(&gi->w2o[2]);
     // normal * gl_WorldToObjectEXT: transpose of the world-to-object 3x3
-    s->normal = norm3(f3(tsn.x * w0.x + tsn.y * w1.x + tsn.z * w2.x, tsn.x * w0.y + tsn.y * w1.y + tsn.z * w2.y,
-                         tsn.x * w0.z + tsn.y * w1.z + tsn.z * w2.z));
+    s->normal = norm_hit(f3(mix_of_three(tsn.x, w0.x, tsn.y, w1.x, tsn.z, w2.x),
+                            mix_of_three(tsn.x, w0.y, tsn.y, w1.y, tsn.z, w2.y),
+                            mix_of_three(tsn.x, w0.z, tsn.y, w1.z, tsn.z, w2.z)));
     const ddgi_material& m = sc.materials[oe.material_index];
     s->albedo = f3(m.base_color[0], m.base_color[1], m.base_color[2]);
     s->emissive = f3(m.emissive[0], m.emissive[1], m.emissive[2]);
@@ -415,6 +486,40 @@ __device__ __forceinline__ bool surface_at(const DeviceScene& sc, float3 origin,
     return true;
 }
 
+__device__ __forceinline__ float3 reflected(float3 dir, float3 normal) {
+    const float k = -2.0f * dot_hit(normal, dir);
+    return f3(fmaf(normal.x, k, dir.x), fmaf(normal.y, k, dir.y), fmaf(normal.z, k, dir.z));
+}
+
+// The shading of surface `s` seen along `dir` from the two lookups' results.
+// Written with explicit multiply-adds here and in the lookups: several kernels
+// shade hits, and all give the same bits.
+__device__ __forceinline__ void shade_from_lookups(const Surface& s, const DeviceLight& L, float3 dir,
+                                                   float3 reflection, float3 indirect, SurfaceShade* out) {
+    out->position = s.position;
+    const float3 normal = s.normal, albedo = s.albedo;
+    const float metal = s.metal, rough = s.rough;
+    const float a[3] = {albedo.x, albedo.y, albedo.z}, r[3] = {reflection.x, reflection.y, reflection.z},
+                i[3] = {indirect.x, indirect.y, indirect.z};
+    float color[3] = {s.emissive.x, s.emissive.y, s.emissive.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float diffuse = __fmul_rn(__fmul_rn(a[c], 1.0f - 0.04f), 1.0f - metal);
+        const float specular = fmaf(0.04f, 1.0f - metal, __fmul_rn(a[c], metal));
+        color[c] = fmaf(i[c], diffuse, fmaf(specular, r[c], color[c]));
+    }
+    out->base = f3(color[0], color[1], color[2]);
+    out->sun = pbr_metallic_roughness(normal, norm_hit(-dir), f3(L.color[0], L.color[1], L.color[2]),
+                                      f3(L.dir[0], L.dir[1], L.dir[2]), albedo, metal, rough);
+    out->fade = L.dir[1] < 0.0f ? 1.0f - clampf(-L.dir[1], 0.0f, 0.1f) / 0.1f : 1.0f;
+}
+// What a hit whose indices are out of range shades to.
+__device__ __forceinline__ void shade_nothing(float3 position, SurfaceShade* out) {
+    out->position = position;
+    out->base = out->sun = f3(0, 0, 0);
+    out->fade = 1.0f;
+}
+
 template <class AV>
 __device__ __forceinline__ bool shade_surface(const DeviceScene& sc, const DeviceGrid& g, const DeviceLight& L,
                                               const uint32_t* states, const AV& at, float3 origin, float3 dir,
@@ -422,27 +527,13 @@ __device__ __forceinline__ bool shade_surface(const DeviceScene& sc, const Devic
                                               SurfaceShade* out, uint32_t* err) {
     Surface s;
     if (!surface_at(sc, origin, dir, t, b1, b2, inst, prim, &s, err)) {
-        out->position = s.position;
-        out->base = out->sun = f3(0, 0, 0);
-        out->fade = 1.0f;
+        shade_nothing(s.position, out);
         return false;
     }
-    out->position = s.position;
-    const float3 position = s.position, normal = s.normal, albedo = s.albedo;
-    const float metal = s.metal, rough = s.rough;
-    float3 color = s.emissive;
-    float3 diffuseColor = albedo * (1.0f - 0.04f) * (1.0f - metal);
-    float3 specularColor = mix3(f3(0.04f, 0.04f, 0.04f), albedo, metal);
-    float3 reflectDir = dir - normal * (2.0f * dot3(normal, dir));
-    const float3 lookups[2] = {reflectDir, normal};
+    const float3 lookups[2] = {reflected(dir, s.normal), s.normal};
     float3 sampled[2];  // reflection, indirect
-    sample_probes_n<2>(position, lookups, -dir, g, states, at, sampled);
-    color = color + specularColor * sampled[0];
-    color = color + sampled[1] * diffuseColor;
-    out->base = color;
-    out->sun = pbr_metallic_roughness(normal, norm3(-dir), f3(L.color[0], L.color[1], L.color[2]),
-                                      f3(L.dir[0], L.dir[1], L.dir[2]), albedo, metal, rough);
-    out->fade = L.dir[1] < 0.0f ? 1.0f - clampf(-L.dir[1], 0.0f, 0.1f) / 0.1f : 1.0f;
+    sample_probes_n<2>(s.position, lookups, -dir, g, states, at, sampled);
+    shade_from_lookups(s, L, dir, sampled[0], sampled[1], out);
     return true;
 }
 

@@ -3,9 +3,10 @@
 //  1. k_primary: closest hit of every probe ray.  Persistent warps; a lane
 //     whose ray finishes is handed the next ray from a global counter, so the
 //     warp keeps its lanes busy instead of waiting for its longest ray.
-//  2. k_shade: one thread per ray record, coalesced: miss -> sky, backface ->
-//     (0, 0.8 t), front face -> shading split around the shadow query; the
-//     front hits are appended (warp-aggregated) to a shadow-ray queue.
+//  2. k_shade_classify, k_shade_front: one thread per ray record, coalesced:
+//     miss -> sky, backface -> (0, 0.8 t), front face -> a queue that is shaded
+//     with one to four lanes per hit, up to the shadow query; the front hits
+//     are appended (warp-aggregated) to a shadow-ray queue.
 //  3. k_shadow: any-hit query of the queued rays toward the sun, persistent
 //     like k_primary; an unshadowed ray gets (base + sun) * fade.
 //
@@ -24,6 +25,7 @@ namespace ddgi {
 namespace {
 
 constexpr int kPersistThreads = kWalkerThreads;  // the walkers' shared-memory stacks assume it
+constexpr uint32_t kShadeBlocksPerSm = 5;  // resident blocks of the front-hit shading
 constexpr unsigned kFull = 0xffffffffu;
 
 // Work item `id` of a grouped order: groups of G = 32 / rpw probes (in perm
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(128) k_shade_classify(DeviceGrid g, DeviceLigh
 // the 1M-triangle terrain update against 373 us at six and 396 us at four; 23,
 // 25 and 22 us for the 65 K hits of a small room.
 template <class AV>
-__global__ void __launch_bounds__(128, 5) k_shade_front(DeviceScene sc, DeviceGrid g, DeviceLight L,
+__global__ void __launch_bounds__(128, kShadeBlocksPerSm) k_shade_front(DeviceScene sc, DeviceGrid g, DeviceLight L,
                                                         const uint32_t* __restrict__ probe_list,
                                                         const float4* __restrict__ dirs,
                                                         const uint32_t* __restrict__ states, AV at, WaveHits hits,
@@ -379,6 +381,60 @@ struct BatchPrimaryJob {
     }
 };
 
+// The same with 2 x PARTS lanes per hit: half of them for each of its two
+// lookups, in which each takes every PARTS-th probe (the rest of the hit is
+// done by all).  With fewer hits than the chip has threads for, the time is one
+// thread's chain of eight probes' loads and quotients, which this shortens:
+// the 65 K hits of 512 probes 26 -> 17 us, 16 K 20 -> 11 us.
+template <int PARTS, class AV>
+__global__ void __launch_bounds__(128, kShadeBlocksPerSm) k_shade_front_split(DeviceScene sc, DeviceGrid g, DeviceLight L,
+                                                              const uint32_t* __restrict__ probe_list,
+                                                              const float4* __restrict__ dirs,
+                                                              const uint32_t* __restrict__ states, AV at,
+                                                              WaveHits hits, const uint32_t* front_count,
+                                                              float4* rays_out, ShadowQueue q, uint32_t* err) {
+    constexpr uint32_t kLanes = 2u * PARTS;
+    after_previous();
+    const uint32_t n = *front_count;
+    if (blockIdx.x * (blockDim.x / kLanes) >= n) return;  // whole block
+    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes, lane = threadIdx.x % kLanes;
+    bool ok = false;
+    Surface s;
+    s.position = s.normal = f3(0, 0, 0);
+    float3 dir = f3(0, 0, 0);
+    uint32_t i = 0;
+    float t = 0.0f;
+    if (k < n) {
+        i = hits.front[k];
+        const uint32_t R = g.rays;
+        const uint32_t slot = i / R, ray = i - slot * R;
+        const float4 th = hits.thit[i];
+        const uint32_t inst = __float_as_uint(th.w), prim = hits.prim[i] & 0x0fffffffu;
+        const uint32_t probe = probe_list ? __ldg(probe_list + slot) : slot;
+        const float4 d4 = __ldg(dirs + ray);
+        dir = f3(d4.x, d4.y, d4.z);
+        t = th.x;
+        ok = surface_at(sc, probe_origin_exact(g, probe), dir, th.x, th.y, th.z, inst, prim, &s, err);
+    }
+    const float3 mine = sample_probes_split<PARTS>(ok, s.position, lane < PARTS ? reflected(dir, s.normal) : s.normal,
+                                                   -dir, g, states, at);
+    const float3 other = f3(__shfl_xor_sync(kFull, mine.x, PARTS), __shfl_xor_sync(kFull, mine.y, PARTS),
+                            __shfl_xor_sync(kFull, mine.z, PARTS));
+    SurfaceShade o;
+    if (lane == 0 && k < n) {
+        if (ok) shade_from_lookups(s, L, dir, mine, other, &o);
+        else shade_nothing(s.position, &o);
+        rays_out[i] = make_float4(o.base.x, o.base.y, o.base.z, t);
+    }
+    const bool enqueue = lane == 0 && ok;
+    const uint32_t qk = warp_append(enqueue, q.count);
+    if (enqueue) {
+        q.idx[qk] = i;
+        q.pos[qk] = make_float4(o.position.x, o.position.y, o.position.z, 0.0f);
+        q.sun[qk] = make_float4(o.sun.x, o.sun.y, o.sun.z, o.fade);
+    }
+}
+
 struct BatchShadowJob {
     static constexpr float kTmin = 0.1f;
     static constexpr uint32_t kMask = 0xFFu;
@@ -508,6 +564,23 @@ uint32_t persistent_blocks(const void* kernel, size_t smem, uint32_t cap_per_sm 
     return (uint32_t)(sms * per);
 }
 
+// Lanes per hit of the front-hit shading for at most `total` hits, from the
+// threads resident at a time (`slots`, 97,280 on 152 SMs).  Rooms of 128 rays a
+// probe, all probes, 1 / 2 / 4 lanes (us):
+//   records      32,768         65,536         98,304         196,608
+//   FP32 atlas   21 / 13 / 13   25 / 17 / 23   27 / 30 / 33   59 / 46 / 54
+//   FP16 atlas   18 / 13 / 12   19 / 15 / 20   20 / 25 / 28   38 / 39 / 46
+// Four lanes win while they fit with the hits' usual share of the records, two
+// while the launch fits in a round and a half.  Beyond that the two-lane form
+// still wins over an FP32 atlas, where one lane's two lookups spill registers
+// (1,048,576 records: 208 / 196 us), until the work done twice costs more
+// (4,194,304: a 6.47 ms update is 0.2 % slower).
+uint32_t shade_lanes(uint32_t total, bool fp16_atlas) {
+    const uint32_t slots = kShadeBlocksPerSm * 128u * sm_count();
+    if (total <= slots / 3u) return 4u;
+    return total <= (fp16_atlas ? slots / 4u * 3u : slots * 16u) ? 2u : 1u;
+}
+
 }  // namespace
 
 namespace {
@@ -530,17 +603,21 @@ cudaError_t wavefront_kernels(const DeviceScene& sc, const DeviceGrid& g, const 
     cudaError_t e = launch_dependent(k_shade_classify, blocks, 128, 0, st, g, L, total, hits, rays_out, hits_out,
                                      counters + 3, dev_count);
     if (e != cudaSuccess) return e;
-    if (fp16_atlas) {
-        AtlasView<ColorTexF16, DepthTexF16> at{{static_cast<const uint2*>(color)},
-                                               {static_cast<const uint32_t*>(depth)}};
-        e = launch_dependent(k_shade_front<decltype(at)>, blocks, 128, 0, st, sc, g, L, probe_list, dirs, states, at,
-                             hits, counters + 3, rays_out, qq, err);
-    } else {
-        AtlasView<ColorTexF32, DepthTexF32> at{{static_cast<const float4*>(color)},
-                                               {static_cast<const float2*>(depth)}};
-        e = launch_dependent(k_shade_front<decltype(at)>, blocks, 128, 0, st, sc, g, L, probe_list, dirs, states, at,
-                             hits, counters + 3, rays_out, qq, err);
-    }
+    const uint32_t lanes = shade_lanes(total, fp16_atlas);
+    const uint32_t shade_blocks = (uint32_t)(((uint64_t)total * lanes + 127) / 128);
+    auto shade = [&](auto at) {
+        auto launch = [&](auto kernel) {
+            return launch_dependent(kernel, shade_blocks, 128, 0, st, sc, g, L, probe_list, dirs, states, at, hits,
+                                    counters + 3, rays_out, qq, err);
+        };
+        if (lanes == 4u) return launch(k_shade_front_split<2, decltype(at)>);
+        if (lanes == 2u) return launch(k_shade_front_split<1, decltype(at)>);
+        return launch(k_shade_front<decltype(at)>);
+    };
+    e = fp16_atlas ? shade(AtlasView<ColorTexF16, DepthTexF16>{{static_cast<const uint2*>(color)},
+                                                               {static_cast<const uint32_t*>(depth)}})
+                   : shade(AtlasView<ColorTexF32, DepthTexF32>{{static_cast<const float4*>(color)},
+                                                               {static_cast<const float2*>(depth)}});
     if (e != cudaSuccess) return e;
     ShadowJob sj{qq, make_float3(L.dir[0], L.dir[1], L.dir[2]), rays_out, hits.prim, 0};
     e = launch_dependent(k_shadow<Stack, Walker>,
