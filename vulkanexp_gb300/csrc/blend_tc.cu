@@ -25,8 +25,8 @@
 // three products hi*hi + hi*lo + lo*hi are accumulated (~16 mantissa bits,
 // below the FP16 atlas store's rounding; BF16 keeps FP32's exponent range,
 // so no scaling is needed).  One thread issues tcgen05.mma (M = 128,
-// K = 16); while a chunk's MMAs run, the next chunks' weights arrive by
-// cp.async and their records into registers.  With 256 accumulator columns
+// K = 16); while a pair of chunks' MMAs run, the next pair's weights arrive by
+// bulk copies and its records into registers.  With 256 accumulator columns
 // two CTAs share an SM.  The epilogue reads the accumulators with
 // tcgen05.ld, normalises (times the reciprocal row sums) through shared
 // memory into texel order, applies hysteresis in the FP32 accumulators
@@ -51,7 +51,7 @@ constexpr int kMinTileProbes = 4;  // smallest tile of a launch that fills less 
 constexpr int kMinRoundTile = 16;  // smallest tile of a launch of several rounds
 constexpr int kRowsPerProbe = 5;
 constexpr int kKChunk = 16;        // rays per shared-memory stage (one K step)
-constexpr int kStages = 4;         // operand stages in the ring
+constexpr int kStages = 4;         // operand stages in the ring: two pairs of chunks
 constexpr int kThreads = 256;
 constexpr uint32_t kSBO = (kKChunk / 8) * 128;  // bytes between 8-row groups
 constexpr uint32_t kLBO = 128;                  // bytes between K-adjacent core matrices
@@ -237,17 +237,22 @@ __host__ __device__ __forceinline__ size_t tc_smem_bytes(uint32_t nc, uint32_t n
 }
 
 // Blend of the tile of a.tile probe slots starting at p0 (< nprobes) by the
-// whole CTA.  Iteration c fills stage c % kStages with chunk c (weights
-// by cp.async, ray operands from registers loaded two iterations before) and
-// issues the MMAs of chunk c - 1, whose weights were copied one iteration
-// before; a stage is refilled once the MMAs that read it (kStages chunks
-// earlier) have signalled its barrier.
+// whole CTA, two chunks at a time.  Iteration p fills its pair of stages with
+// the chunks' ray operands (from registers loaded an iteration before) and
+// issues their MMAs once their weights are there: a bulk copy per chunk, asked
+// for an iteration ahead by the thread that issues the MMAs.  The stages are
+// refilled once the MMAs that read them (two pairs earlier) have signalled
+// their barrier.  An iteration's time is the proxy fence, which waits for the
+// thread's loads and cp.async copies under way: one chunk an iteration with
+// records and 16-byte weight copies in flight across the fence took 1,300
+// cycles a chunk, this takes 1,000.
 __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0, const uint32_t nprobes) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t s_bar[kStages];
+    __shared__ uint64_t s_bar[2];   // a pair of stages: its MMAs are done
+    __shared__ uint64_t s_full[2];  // its weights are there
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_oor[kTileProbes], s_maxc[kTileProbes];
-    __shared__ float s_rinv[512];       // 1 / row sum of the weights (1 where the sum is <= 1e-3)
+    __shared__ __align__(16) float s_rinv[512];       // 1 / row sum of the weights (1 where the sum is <= 1e-3)
     __shared__ int2 s_org[kTileProbes];  // atlas tile (x, y) of each probe, in tiles; x < 0: none
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -264,7 +269,11 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
     auto stage_b = [&](uint32_t c) { return smem + (c % kStages) * sbytes + 2 * kAPart; };
 
     if (warp == 0) tc::tmem_alloc(&s_tmem, cols);
-    if (tid < kStages) tc::mbar_init(&s_bar[tid], 1);
+    if (tid < 2) {
+        tc::mbar_init(&s_bar[tid], 1);
+        tc::mbar_init(&s_full[tid], 1);
+        tc::fence_mbar_init();
+    }
     if (tid < kTileProbes) {
         s_maxc[tid] = 0u;
         s_oor[tid] = 0u;
@@ -281,16 +290,16 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
         }
         s_org[tid] = o;
     }
-    for (uint32_t i = tid; i < a.Nd + a.Nc; i += kThreads) {
-        const float sum = a.rowsum[i];
-        s_rinv[i] = sum > 1e-3f ? 1.0f / sum : 1.0f;
-    }
     // A rows tile * 5 .. 127 stay zero in every stage
     const uint32_t zrows = 128u - a.tile * kRowsPerProbe;
     for (uint32_t i = tid; i < kStages * 2 * zrows * (kKChunk / 8); i += kThreads) {
         const uint32_t kg = i % (kKChunk / 8), r = a.tile * kRowsPerProbe + (i / (kKChunk / 8)) % zrows;
         const uint32_t part = (i / (zrows * (kKChunk / 8))) % 2, st = i / (2 * zrows * (kKChunk / 8));
         *reinterpret_cast<uint4*>(smem + st * sbytes + part * kAPart + canon_off(r, kg)) = make_uint4(0, 0, 0, 0);
+    }
+    for (uint32_t i = tid; i < a.Nd + a.Nc; i += kThreads) {
+        const float sum = a.rowsum[i];
+        s_rinv[i] = sum > 1e-3f ? 1.0f / sum : 1.0f;
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -302,59 +311,58 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
     const bool builder = pl < a.tile;
     const bool live = builder && pl < np;
     const float4* prec = a.rays + (size_t)(p0 + (live ? pl : 0u)) * R;
-    float4 va[2], vb[2];  // records of the even / odd chunks in flight
-    auto load = [&](float4* v, uint32_t c) {
+    float4 v[4];  // the next pair's records: two of each chunk
+    auto load = [&](uint32_t c0) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const uint32_t r = c * kKChunk + j * 2 + e;
+        for (uint32_t e = 0; e < 4; ++e) {
+            const uint32_t r = (c0 + (e >> 1)) * kKChunk + j * 2 + (e & 1u);
             v[e] = live && r < R ? prec[r] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
-    load(va, 0);
-    load(vb, 1);
+    load(0);
     uint32_t oor = 0;
     const uint32_t N = a.Nd + a.Nc;
     const uint32_t id_all = tc::idesc_bf16_f32(128, N), id_d = tc::idesc_bf16_f32(128, a.Nd),
                    id_c = tc::idesc_bf16_f32(128, a.Nc);
     bool ok = true;
-    uint32_t waited = 0;  // chunk whose MMAs a completion wait was for (the drain's target on a timeout)
-    int last = -1;        // the last chunk whose MMAs were issued
-    for (uint32_t c = 0; c <= a.nchunks; ++c) {
-        if (c < a.nchunks) {
-            if (c >= (uint32_t)kStages) {  // the MMAs of chunk c - kStages read this stage
-                const uint32_t old = c - kStages;
-                const bool done = tc::mbar_wait(&s_bar[old % kStages], (old / kStages) & 1u, kWaitLimitNs);
-                tc::fence_after_sync();
-                if (!__syncthreads_and(done)) {
-                    ok = false;
-                    waited = old;
-                    break;
-                }
-            }
-            {   // weights of chunk c
-                const uint4* src = a.wchunks + (size_t)c * b16;
-                uint4* dst = reinterpret_cast<uint4*>(stage_b(c));
-                for (uint32_t i = tid; i < b16; i += kThreads) tc::cp_async16(dst + i, src + i);
-                tc::cp_async_commit();
-            }
-            if (builder) {  // A rows (r, g, b, d, d^2) of this thread's probe, 2 rays: a quarter core-matrix row
-                float4 v[2];
+    const uint32_t npairs = (a.nchunks + 1) / 2;
+    uint32_t copied = 0;      // pairs whose weights were asked for (thread 0)
+    bool feeding = tid == 0;  // thread 0, until a wait of its own runs out
+    auto copy_weights = [&]() {
+        const uint32_t c = 2 * copied, n = min(2u, a.nchunks - c);
+        uint64_t* bar = &s_full[copied & 1u];
+        tc::expect_bytes(bar, n * (uint32_t)bbytes);
+        for (uint32_t k = 0; k < n; ++k)
+            tc::bulk_load(stage_b(c + k), a.wchunks + (size_t)(c + k) * b16, (uint32_t)bbytes, bar);
+        ++copied;
+    };
+    if (feeding)
+        while (copied < min(2u, npairs)) copy_weights();
+    for (uint32_t p = 0; p < npairs; ++p) {
+        bool done = true;
+        if (p >= 2) {  // the MMAs of pair p - 2 read these stages
+            done = tc::mbar_wait(&s_bar[p & 1u], ((p - 2) >> 1) & 1u, kWaitLimitNs);
+            tc::fence_after_sync();
+        }
+        if (builder && done) {  // A rows (r, g, b, d, d^2) of this thread's probe, 2 rays: a quarter core-matrix row
 #pragma unroll
-                for (int e = 0; e < 2; ++e) v[e] = (c & 1u) ? vb[e] : va[e];
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint32_t c = 2 * p + h;
+                const float4 x = v[2 * h], y = v[2 * h + 1];
                 float dep[2];
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
+                for (uint32_t e = 0; e < 2; ++e) {
                     const uint32_t r = c * kKChunk + j * 2 + e;
-                    const float wv = v[e].w;
+                    const float wv = e ? y.w : x.w;
                     if (live && r < R && (wv < 0.0f || wv > cell)) ++oor;
                     float dd = fminf(cell, wv);
                     if (dd < 0.0f) dd = cell;
                     dep[e] = live && r < R ? dd : 0.0f;
                 }
                 uint32_t w[5][2];
-                w[0][0] = pack2(v[0].x, v[1].x, &w[0][1]);
-                w[1][0] = pack2(v[0].y, v[1].y, &w[1][1]);
-                w[2][0] = pack2(v[0].z, v[1].z, &w[2][1]);
+                w[0][0] = pack2(x.x, y.x, &w[0][1]);
+                w[1][0] = pack2(x.y, y.y, &w[1][1]);
+                w[2][0] = pack2(x.z, y.z, &w[2][1]);
                 w[3][0] = pack2(dep[0], dep[1], &w[3][1]);
                 w[4][0] = pack2(dep[0] * dep[0], dep[1] * dep[1], &w[4][1]);
                 uint8_t* sa = stage_a(c);
@@ -366,47 +374,50 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
                                                      canon_off(pl * kRowsPerProbe + ch, j >> 2) + (j & 3u) * 4u) =
                             w[ch][part];
             }
-            if (c + 2 < a.nchunks) {  // records two chunks ahead
-                if (c & 1u) load(vb, c + 2);
-                else load(va, c + 2);
-            }
         }
-        if (c >= 1) {  // the MMAs of chunk c - 1 (its weights were copied an iteration ago)
-            if (c < a.nchunks) tc::cp_async_wait_group<1>();
-            else tc::cp_async_wait_group<0>();
-            tc::fence_proxy_async();
-            __syncthreads();
-            const uint32_t m = c - 1;
-            if (tid == 0 && !a.stall) {
+        tc::fence_proxy_async();  // waits for this thread's loads too: none are under way here
+        if (p + 1 < npairs) load(2 * p + 2);
+        if (!__syncthreads_and(done)) {
+            ok = false;
+            break;
+        }
+        if (feeding && !a.stall) {
+            feeding = tc::mbar_wait(&s_full[p & 1u], (p >> 1) & 1u, kWaitLimitNs);
+            if (feeding) {
                 tc::fence_after_sync();
-                const uint32_t aH = tc::smem_u32(stage_a(m)), aL = aH + kAPart;
-                const uint32_t bH = tc::smem_u32(stage_b(m)), bL = bH + N * (kKChunk * 2);
-                // hi*hi + hi*lo + lo*hi, K = 16 per instruction
-                const uint32_t a_[3] = {aH, aH, aL}, b_[3] = {bH, bL, bH};
+                for (uint32_t c = 2 * p; c < min(2 * p + 2, a.nchunks); ++c) {
+                    const uint32_t aH = tc::smem_u32(stage_a(c)), aL = aH + kAPart;
+                    const uint32_t bH = tc::smem_u32(stage_b(c)), bL = bH + N * (kKChunk * 2);
+                    // hi*hi + hi*lo + lo*hi, K = 16 per instruction
+                    const uint32_t a_[3] = {aH, aH, aL}, b_[3] = {bH, bL, bH};
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    const uint32_t acc = (m > 0 || q > 0) ? 1u : 0u;
-                    const uint64_t ad = tc::smem_desc(a_[q], kLBO, kSBO);
-                    if (!split) {
-                        tc::mma_bf16(tmem, ad, tc::smem_desc(b_[q], kLBO, kSBO), id_all, acc);
-                    } else {
-                        tc::mma_bf16(tmem, ad, tc::smem_desc(b_[q], kLBO, kSBO), id_d, acc);
-                        tc::mma_bf16(tmem + 256u, ad, tc::smem_desc(b_[q] + a.Nd * (kKChunk * 2), kLBO, kSBO), id_c,
-                                     acc);
+                    for (int q = 0; q < 3; ++q) {
+                        const uint32_t acc = (c > 0 || q > 0) ? 1u : 0u;
+                        const uint64_t ad = tc::smem_desc(a_[q], kLBO, kSBO);
+                        if (!split) {
+                            tc::mma_bf16(tmem, ad, tc::smem_desc(b_[q], kLBO, kSBO), id_all, acc);
+                        } else {
+                            tc::mma_bf16(tmem, ad, tc::smem_desc(b_[q], kLBO, kSBO), id_d, acc);
+                            tc::mma_bf16(tmem + 256u, ad, tc::smem_desc(b_[q] + a.Nd * (kKChunk * 2), kLBO, kSBO),
+                                         id_c, acc);
+                        }
                     }
                 }
-                tc::commit(&s_bar[m % kStages]);
+                tc::commit(&s_bar[p & 1u]);
+                // the stages that pair p - 1's MMAs have read take the weights of pair p + 1
+                if (p >= 1 && copied < npairs) {
+                    feeding = tc::mbar_wait(&s_bar[(p - 1) & 1u], ((p - 1) >> 1) & 1u, kWaitLimitNs);
+                    if (feeding) copy_weights();
+                }
             }
-            last = (int)m;
-            __syncwarp();
         }
+        __syncwarp();
     }
-    if (ok && last >= 0) {  // the last chunk's MMAs (a commit tracks every earlier MMA too)
-        const uint32_t m = (uint32_t)last;
-        const bool done = tc::mbar_wait(&s_bar[m % kStages], (m / kStages) & 1u, kWaitLimitNs);
+    const uint32_t last = npairs - 1;
+    if (ok) {  // the last pair's MMAs (a commit tracks every earlier MMA too)
+        const bool done = tc::mbar_wait(&s_bar[last & 1u], (last >> 1) & 1u, kWaitLimitNs);
         tc::fence_after_sync();
         ok = __syncthreads_and(done);
-        waited = m;
     }
     if (live && oor) atomicAdd(&s_oor[pl], oor);
 
@@ -416,11 +427,16 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
         // in flight; a preempted CTA's MMAs finish once it runs again), then
         // release the tensor memory: a CTA must not exit holding it
         if (tid == 0) raise_error(a.err, DEV_WAIT_TIMEOUT);
-        if (!a.stall && last >= 0) {  // the stall hook issued none
-            const uint32_t m = (uint32_t)last;
-            tc::mbar_wait(&s_bar[m % kStages], (m / kStages) & 1u, kDrainLimitNs);
-        }
-        (void)waited;
+        // and no copy may be under way when the CTA's shared memory goes to another
+        if (tid == 0)
+            for (uint32_t k = 0; k < 2; ++k) {
+                if (k < copied) {
+                    const uint32_t p = copied - 1 - k;
+                    tc::mbar_wait(&s_full[p & 1u], (p >> 1) & 1u, kDrainLimitNs);
+                    if (!a.stall) tc::mbar_wait(&s_bar[p & 1u], (p >> 1) & 1u, kDrainLimitNs);
+                }
+            }
+        __syncthreads();
     } else {
         // epilogue 1: accumulators -> normalised values in shared staging,
         // texel-major: S_c[probe][texel][r, g, b], S_d[probe][texel][d, d^2]
@@ -439,19 +455,32 @@ __device__ __forceinline__ void blend_tc_tile(const TcArgs& a, const uint32_t p0
             float vv[16];
             tc::tmem_ld16(lane_base + col0, vv);
             if (!rvalid) continue;
+            // the sixteen scales before the first store: a load behind a store
+            // to shared memory waits for it (this loop 6,400 -> 3,700 cycles of
+            // a CTA)
+            float4 sc[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sc[i] = reinterpret_cast<const float4*>(s_rinv)[s * 4 + i];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                vv[4 * i] *= sc[i].x;
+                vv[4 * i + 1] *= sc[i].y;
+                vv[4 * i + 2] *= sc[i].z;
+                vv[4 * i + 3] *= sc[i].w;
+            }
             if (depth && ch >= 3) {
                 float* dst = S_d + rp * ntd * 2 + (ch - 3);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const uint32_t u = s * 16 + i;
-                    if (u < ntd) dst[u * 2] = vv[i] * s_rinv[u];
+                    if (u < ntd) dst[u * 2] = vv[i];
                 }
             } else if (!depth && ch < 3) {
                 float* dst = S_c + rp * ntc * 3 + ch;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const uint32_t t = (s - steps_d) * 16 + i;
-                    if (t < ntc) dst[t * 3] = vv[i] * s_rinv[a.Nd + t];
+                    if (t < ntc) dst[t * 3] = vv[i];
                 }
             }
         }
