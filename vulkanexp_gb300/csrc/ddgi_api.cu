@@ -1281,6 +1281,7 @@ ddgi_status ddgi_update_instances(ddgi_ctx* ctx, const uint32_t* ids, const floa
             return fail(ctx, DDGI_ERR_UNSUPPORTED, "rebuilt top level too deep (%u levels)", dtop);
         S.depth_tlas = dtop;
         S.stack_cap = cap;
+        CK(launch_walk_nodes(S.nodes + S.tlas_root, ni > 1 ? ni - 1 : 1, S.walk + S.tlas_root, st), "walk nodes");
     } else {
         // refit: same topology, new leaf boxes, boxes recomputed bottom-up
         std::vector<GpuInstance> leaf(ni);
@@ -1297,11 +1298,10 @@ ddgi_status ddgi_update_instances(ddgi_ctx* ctx, const uint32_t* ids, const floa
         CK(cudaMemcpyAsync(S.leaf_lo, llo.data(), sizeof(float4) * ni, cudaMemcpyHostToDevice, st), "upload");
         CK(cudaMemcpyAsync(S.leaf_hi, lhi.data(), sizeof(float4) * ni, cudaMemcpyHostToDevice, st), "upload");
         CK(lbvh_refit_top(S.nodes, S.tlas_root, S.leaf_lo, S.leaf_hi, ni, S.leaf_parent, S.node_parent, S.refit_flags,
-                          S.sub_lo, S.sub_hi, ctx->err, st),
+                          S.sub_lo, S.sub_hi, S.walk, ctx->err, st),
            "top-level refit");
         // the host vectors above are staged by the copies before they return
     }
-    CK(launch_walk_nodes(S.nodes + S.tlas_root, ni > 1 ? ni - 1 : 1, S.walk + S.tlas_root, st), "walk nodes");
     {
         ddgi_status ws = refresh_wide_top(ctx, st);
         if (ws != DDGI_OK) return ws;

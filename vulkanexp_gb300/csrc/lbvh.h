@@ -37,10 +37,11 @@ cudaError_t gather_mesh_tris(const float4* pos, const uint32_t* indices, uint32_
 // Refit of a top-level tree whose topology is kept: new boxes for its n
 // leaf slots (leaf order); leaf_parent[s] / node_parent[k] = parent node
 // (relative to node_base) << 1 | side, 0xFFFFFFFF for the root; flags
-// (n - 1 entries) and sub_lo/sub_hi (2 (n - 1) entries) are scratch.
+// (n - 1 entries) and sub_lo/sub_hi (2 (n - 1) entries) are scratch.  The
+// nodes' copies in the walkers' form are renewed too (walk: indexed like nodes).
 cudaError_t lbvh_refit_top(BvhNode* nodes, int node_base, const float4* leaf_lo, const float4* leaf_hi, uint32_t n,
                            const uint32_t* leaf_parent, const uint32_t* node_parent, uint32_t* flags, float4* sub_lo,
-                           float4* sub_hi, uint32_t* err, cudaStream_t st);
+                           float4* sub_hi, WalkNode* walk, uint32_t* err, cudaStream_t st);
 
 // The `n` nodes from `nodes` in the persistent walkers' form.
 cudaError_t launch_walk_nodes(const BvhNode* nodes, uint32_t n, WalkNode* out, cudaStream_t st);
