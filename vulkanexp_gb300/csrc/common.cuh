@@ -83,8 +83,9 @@ static_assert(sizeof(BvhNode) == 64, "node is 64 bytes");
 // instructions, and the references between them:
 //   c0.x c0.y | c1.x c1.y | c0.z c1.z | ref0 ref1
 //   h0.x h0.y | h1.x h1.y | h0.z h1.z | unused
-// A box that is never hit has half extents of -infinity, one that overflowed
-// +infinity about zero.
+// A box that is never hit has half extents of -infinity, along an axis where
+// it reaches beyond kWalkReach +infinity about zero (never pruned there).
+constexpr float kWalkReach = 0x1p60f;
 struct __align__(32) WalkNode {
     float c0[2], c1[2], cz[2];
     int32_t ref[2];

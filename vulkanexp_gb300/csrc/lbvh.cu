@@ -427,14 +427,13 @@ namespace {
 // One child's interval along one axis as centre and half extent: the half
 // extent is rounded up from the farther plane, so the interval holds [lo, hi].
 __device__ __forceinline__ void centre_half(float lo, float hi, float* c, float* h) {
-    if (!(lo <= hi)) {  // never hit
+    if (lo > hi) {  // never hit
         *c = 0.0f;
         *h = -INFINITY;
-        return;
-    }
-    *c = 0.5f * lo + 0.5f * hi;
-    *h = fmaxf(__fsub_ru(hi, *c), __fsub_ru(*c, lo));
-    if (!isfinite(*c) || !isfinite(*h)) {  // a plane overflowed: always hit
+    } else if (lo >= -kWalkReach && hi <= kWalkReach) {
+        *c = 0.5f * lo + 0.5f * hi;
+        *h = fmaxf(__fsub_ru(hi, *c), __fsub_ru(*c, lo));
+    } else {  // too far for the box test's products, or not a number: always hit
         *c = 0.0f;
         *h = INFINITY;
     }

@@ -218,11 +218,16 @@ struct WorldRay {
 // direction and their magnitudes, paired (x, y) and (z, z) for the packed
 // instructions.  The reciprocal is the approximate one (1 ulp); box distances
 // carry a margin for it (kSlab).
+//
+// A direction component below 2^-66 stands in as +-2^-66.  Over a distance t
+// that moves the ray by at most 2^-66 t, within the 1e-7 by which every box is
+// enlarged at least for t up to 7e12, where the triangle test's own products
+// pass the largest float.  And a centre's distance times the reciprocal stays
+// finite for every box that has a finite form (kWalkReach).
 struct BoxRay {
     uint64_t oxy, ozz, ixy, izz, axy, azz;
     __device__ __forceinline__ void set(float3 o, float3 d) {
-        const float x = rcp(d.x != 0.0f ? d.x : 1e-30f), y = rcp(d.y != 0.0f ? d.y : 1e-30f),
-                    z = rcp(d.z != 0.0f ? d.z : 1e-30f);
+        const float x = rcp(d.x), y = rcp(d.y), z = rcp(d.z);
         oxy = pack2(-o.x, -o.y);
         ozz = pack2(-o.z, -o.z);
         ixy = pack2(x, y);
@@ -238,7 +243,7 @@ struct BoxRay {
     }
     static __device__ __forceinline__ float rcp(float v) {
         float r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(copysignf(fmaxf(fabsf(v), 0x1p-66f), v)));
         return r;
     }
 };
@@ -246,16 +251,21 @@ struct BoxRay {
 // A box [c - h, c + h] is entered at (c - o) / d - h / |d| and left at
 // (c - o) / d + h / |d| along each axis: an addition and a product for the
 // centre and one multiply-add for either plane, with no minimum or maximum to
-// tell the planes apart, and two values per packed instruction (20 instructions
-// for a node's two boxes against 44 for lower and upper planes).
+// tell the planes apart, and two values per packed instruction (9 packed, 6
+// scalar multiply-adds, 8 minima and maxima and 2 scalings for a node's two
+// boxes, against 44 instructions for lower and upper planes).
 //
 // Rounding: a plane's distance is off by at most 3 x 2^-23 of the centre's
 // distance, plus the reciprocal's 2^-23.  Seen from outside a box that is
 // relative to the distance itself, and kSlab, which scales the exit distance
 // before it is compared with the entry, covers it sixteen-fold; near or inside
 // a box it is relative to the box's own extent, and the builders enlarge
-// every box by 1e-5 of that, 84 times the error.  So a box that holds a hit is
-// never missed.
+// every box by 1e-5 of that, 84 times the error.  Range: |c| <= 2^60, and a
+// product (c - o) / d that overflows (|c - o| >= 2^62, by BoxRay's 2^66) belongs
+// to a box that starts beyond t = 2^127.  Boxes that reach further than 2^60 have
+// an infinite extent about zero, which prunes nothing: the entry is -infinity
+// and the exit +infinity, or NaN, which the minima and maxima pass over.  So a
+// box that holds a hit is never missed.
 constexpr float kSlab = 1.00001f;
 
 // Both boxes of a node: hit or not, and whether the second comes first, by
