@@ -530,9 +530,11 @@ void instance_world_box(const float* transform, const float* ml, const float* mh
 }
 
 // Top level over S.inst_lo/inst_hi (caller order) at nodes[node_base ...]:
-// the LBVH, the instance records in leaf order, the leaf boxes and the
-// parent links that a later refit needs.  Scratch for ni primitives; the
-// top-level depth goes to depth_dev[0] (which must hold 1 on entry).
+// the tree, the instance records in leaf order, the leaf boxes and the
+// parent links that a later refit needs, and the nodes' copies in the walkers'
+// form (whatever the caller does about the depth, both traversals see the same
+// tree).  Scratch for ni primitives; the top-level depth goes to depth_dev[0]
+// (which must hold 1 on entry).
 ddgi_status build_top_level(ddgi_ctx* ctx, uint64_t node_base, void* scratch, float4* box_lo, float4* box_hi,
                             uint32_t* sorted, uint32_t* depth_dev, cudaStream_t st) {
     SceneBuffers& S = ctx->scene;
@@ -620,6 +622,7 @@ ddgi_status build_top_level(ddgi_ctx* ctx, uint64_t node_base, void* scratch, fl
     CK(cudaMemcpyAsync(S.leaf_hi, lhi.data(), sizeof(float4) * ni, cudaMemcpyHostToDevice, st), "upload");
     CK(cudaMemcpyAsync(S.leaf_parent, lp.data(), sizeof(uint32_t) * ni, cudaMemcpyHostToDevice, st), "upload");
     CK(cudaMemcpyAsync(S.node_parent, np.data(), sizeof(uint32_t) * inner, cudaMemcpyHostToDevice, st), "upload");
+    CK(launch_walk_nodes(S.nodes + node_base, inner, S.walk + node_base, st), "walk nodes");
     S.tlas_root = (int32_t)node_base;
     return DDGI_OK;
 }
@@ -1187,8 +1190,9 @@ ddgi_status ddgi_scene_build(ddgi_ctx* ctx, const ddgi_scene_desc* d, ddgi_strea
             return ls;
         }
     }
-    {
-        cudaError_t e = launch_walk_nodes(S.nodes, (uint32_t)S.node_count, S.walk, st);
+    {   // the mesh trees' nodes (the top level has its copies)
+        const uint64_t n = S.tlas_root >= 0 ? (uint64_t)S.tlas_root : S.node_count;
+        cudaError_t e = launch_walk_nodes(S.nodes, (uint32_t)n, S.walk, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the build is complete on return
         if (e != cudaSuccess) {
             free_scene(ctx->scene);
@@ -1281,7 +1285,6 @@ ddgi_status ddgi_update_instances(ddgi_ctx* ctx, const uint32_t* ids, const floa
             return fail(ctx, DDGI_ERR_UNSUPPORTED, "rebuilt top level too deep (%u levels)", dtop);
         S.depth_tlas = dtop;
         S.stack_cap = cap;
-        CK(launch_walk_nodes(S.nodes + S.tlas_root, ni > 1 ? ni - 1 : 1, S.walk + S.tlas_root, st), "walk nodes");
     } else {
         // refit: same topology, new leaf boxes, boxes recomputed bottom-up
         std::vector<GpuInstance> leaf(ni);
