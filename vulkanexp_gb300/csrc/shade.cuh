@@ -102,8 +102,20 @@ __device__ __forceinline__ float3 norm_hit(float3 a) {
 }
 __device__ __forceinline__ float sqrt_approx(float v) {  // within 2^-23 relative (PTX sqrt.approx)
     float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
+}
+// The same of three radiances.  The form that takes subnormal numbers costs
+// three instructions more a root, which the 24 roots of a lookup would feel (a
+// 1920x1080 final gather 91 us against 87), so it is kept for them.
+__device__ __forceinline__ void sqrt_approx3(const float (&v)[3], float (&r)[3]) {
+    if (fmin3(v[0], v[1], v[2]) < 0x1p-126f) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r[k] = sqrt_approx(v[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r[k]) : "f"(v[k]));
+    }
 }
 
 // sphere_to_oct_uv (common.cuh) with one reciprocal for its quotients.  Each
@@ -241,8 +253,10 @@ __device__ __forceinline__ void probe_weights(const CellProbe& p, float3 bv, flo
     }
     const float dist = sqrt_approx(d2);
     const float variance = fabsf(fmaf(m[0], m[0], -m[1]));
-    const float dm = fmaxf(dist - m[0], 0.0001f);
-    const float cheb = __fdividef(variance, fmaf(dm, dm, variance));
+    // the quotient of a sixteenth of either side, which has the same bits: the
+    // approximate division gives 0 for a divisor above 2^126
+    const float dm = __fmul_rn(fmaxf(dist - m[0], 0.0001f), 0.25f), part = __fmul_rn(variance, 0.0625f);
+    const float cheb = __fdividef(part, fmaf(dm, dm, part));
     w = __fmul_rn(w, (dist <= m[0]) ? 1.0f : fmaxf(__fmul_rn(__fmul_rn(cheb, cheb), cheb), 0.0f));
     w = fmaxf(0.000001f, w);
     const float crush = 0.2f;
@@ -276,9 +290,10 @@ __device__ __forceinline__ ProbeShare probe_share(const CellProbe& p, float3 bia
     ProbeShare x;
     probe_weights(p, p.at - biasedPosition, normal, at.depth, s, g, &x.weight, &x.fallback);
     const float w11 = __fmul_rn(t.ax, t.ay), w10 = t.ax - w11, w01 = t.ay - w11, w00 = 1.0f - t.ax - w01;
+    float c[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-        x.r[k] = sqrt_approx(fmaf(w11, c11[k], fmaf(w01, c01[k], fmaf(w10, c10[k], __fmul_rn(w00, c00[k])))));
+    for (int k = 0; k < 3; ++k) c[k] = fmaf(w11, c11[k], fmaf(w01, c01[k], fmaf(w10, c10[k], __fmul_rn(w00, c00[k]))));
+    sqrt_approx3(c, x.r);
     return x;
 }
 
@@ -321,9 +336,13 @@ struct LookupSum {
 // (2 ulp, far below the cancellation in the variance), and the eight states
 // are loaded together.  Against the
 // reference's expressions as written: a 1920x1080 final gather over a 16-bit
-// atlas 141 -> 86 us (1,980 warp instructions a warp before), 643x361 over an
-// FP32 atlas 50 -> 38 us, the shading of 65 K hits 39 -> 24 us and of an
-// update's 2.6 M 518 -> 375 us; distance from 64 bits as before (4e-7).
+// atlas 141 -> 87 us (1,980 warp instructions a warp before), 643x361 over an
+// FP32 atlas 50 -> 37 us, the shading of 65 K hits 39 -> 24 us and of an
+// update's 2.6 M 518 -> 375 us.  Distance from a 64-bit evaluation, root mean
+// square of six gathers over 16- and 32-bit atlases: 4.0e-7, 4.8e-7, 5.5e-7,
+// 6.7e-7, 1.1e-6 and 1.3e-5 (a probe's visibility jumping), before 4.0e-7,
+// 4.9e-7, 5.5e-7, 8.2e-7, 1.2e-6 and 1.3e-5.  With correctly rounded roots and
+// quotients it is the same to three digits and the 1920x1080 gather 112 us.
 template <int NQ, class AV>
 __device__ void sample_probes_n(float3 position, const float3 (&normal)[NQ], float3 toCamera, const DeviceGrid& g,
                                 const uint32_t* states, const AV& at, float3 (&result)[NQ]) {
