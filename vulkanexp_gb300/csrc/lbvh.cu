@@ -507,9 +507,12 @@ __global__ void k_refit_top(BvhNode* nodes, int node_base, const float4* lo_in, 
 // is the climb from the deepest leaf, a level after another: through global
 // memory a level is three dependent round trips and two fences, here a few
 // hundred cycles (1,000 instances: 20 us, 2.4 us for the copies' kernel and a
-// clear of the flags -> 16 us; a frame that moves 64 of them 314 -> 305 us).  The
-// limit is what shared memory holds at 56 bytes an instance.
-constexpr uint32_t kBlockRefit = 4096;
+// clear of the flags -> 16 us; a frame that moves 64 of them 314 -> 305 us).  One
+// block has 1,024 threads, so past that each climbs from two leaves and more in
+// turn, while many blocks do not slow down.  One block against many and the
+// copies' kernel, without the clear (us): 256 instances 9 / 24, 1,000 16 / 30,
+// 1,500 23 / 29, 2,048 27 / 32, 3,000 40 / 33, 4,096 48 / 32.
+constexpr uint32_t kBlockRefit = 2048;
 constexpr uint32_t kRefitThreads = 1024;
 __host__ __device__ constexpr size_t refit_smem(uint32_t n) { return (size_t)(n - 1) * (2 * 6 * 4 + 4 + 4); }
 
