@@ -129,12 +129,14 @@ __device__ __forceinline__ void load_pairs(const float* p, uint64_t (&v)[TP / 2]
     }
 }
 
-// Blend of probes p0 .. p0 + np - 1 (slots of `rays`) by one block.
+// Blend of probes p0 .. p0 + np - 1 (slots of `rays`) by one block.  The records
+// and the weights come from kernels that can still be running when this one is
+// set up, so their pointers are not declared to be read-only throughout.
 template <uint32_t TP>
-__device__ __forceinline__ void blend_probes_shared(const DeviceGrid& g, const uint32_t* __restrict__ probe_list,
-                                                    uint32_t p0, uint32_t np, const float4* __restrict__ rays,
-                                                    const float* __restrict__ W, const float* __restrict__ wsum,
-                                                    uint32_t* states, float4* color, float2* depth, const float hy) {
+__device__ __forceinline__ void blend_probes_shared(const DeviceGrid& g, const uint32_t* probe_list, uint32_t p0,
+                                                    uint32_t np, const float4* rays, const float* W,
+                                                    const float* wsum, uint32_t* states, float4* color,
+                                                    float2* depth, const float hy) {
     extern __shared__ float4 s_dyn[];
     float* const s_rec = reinterpret_cast<float*>(s_dyn);  // [R][record_words]: colour, clamped depth
     __shared__ uint32_t s_max_change[TP], s_out_of_range[TP], s_probe[TP];
