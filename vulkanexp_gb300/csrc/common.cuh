@@ -4,7 +4,9 @@
 // transform, watertight triangle test, hit position) is written with
 // explicitly rounded intrinsics (__fmul_rn / __fadd_rn / __fdiv_rn), so that
 // no multiply-add is contracted and the result is bit-identical to a
-// separately-rounded CPU evaluation.  The shading math below it may contract.
+// separately-rounded CPU evaluation.  The vector helpers below may contract;
+// the atlas lookups and the shading of hits write their multiply-adds out
+// (shade.cuh), so that every kernel that shades gives the same bits.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -396,7 +398,7 @@ __device__ __forceinline__ BvhNode load_node(const BvhNode* nodes, int i) {
 }
 
 // ---------------------------------------------------------------------------
-// float3 helpers (shading; contraction allowed)
+// float3 helpers (contraction allowed)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float3 f3(float a, float b, float c) { return make_float3(a, b, c); }
 __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }
@@ -409,10 +411,8 @@ __device__ __forceinline__ float3 operator-(float3 a) { return f3(-a.x, -a.y, -a
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ float len3(float3 a) { return sqrtf(dot3(a, a)); }
 __device__ __forceinline__ float3 norm3(float3 a) { return a * (1.0f / len3(a)); }
-__device__ __forceinline__ float3 abs3(float3 a) { return f3(fabsf(a.x), fabsf(a.y), fabsf(a.z)); }
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fminf(fmaxf(v, lo), hi); }
 __device__ __forceinline__ float3 mix3(float3 a, float3 b, float t) { return a * (1.0f - t) + b * t; }
-__device__ __forceinline__ float gsign(float v) { return v > 0.0f ? 1.0f : (v < 0.0f ? -1.0f : 0.0f); }
 __device__ __forceinline__ float sign_nz(float v) { return v >= 0.0f ? 1.0f : -1.0f; }
 
 // common.glsl:4
@@ -430,21 +430,6 @@ __device__ __forceinline__ float3 oct_decode(float ox, float oy) {
     return norm3(v);
 }
 
-// irradiance.glsl:119-138
-__device__ __forceinline__ float2 sphere_to_oct_uv(float3 d) {
-    float3 oct = f3(gsign(d.x), gsign(d.y), gsign(d.z));
-    float sum = dot3(d, oct);
-    float3 o = f3(d.x / sum, d.y / sum, d.z / sum);
-    if (o.z < 0.0f) {
-        float3 a = abs3(o);
-        float nx = oct.x * (1.0f - a.y);
-        float ny = oct.y * (1.0f - a.x);
-        o.x = nx;
-        o.y = ny;
-    }
-    return make_float2(o.x * 0.5f + 0.5f, o.y * 0.5f + 0.5f);
-}
-
 // Texel-centre scale of probesUpdate.glsl:33-42 for interior side n.
 __host__ __device__ __forceinline__ float texel_scale(uint32_t n) {
     if (n == 6) return 0.33333f;
@@ -455,40 +440,13 @@ __host__ __device__ __forceinline__ float texel_scale(uint32_t n) {
 // REPEAT addressing of texel index i on an axis of n texels.  Sample
 // coordinates in [-0.5, 1.5] give indices in [-n, 2n), which one add or
 // subtract brings into range; anything else takes the remainder (the same
-// integer either way, without a division on the common path).
+// integer either way, without a division on the common path).  The lookups'
+// taps stay inside a probe's tile and need no wrapping (atlas_tap in shade.cuh).
 __host__ __device__ __forceinline__ int wrap_repeat(int i, int n) {
     if (i < 0) i += n;
     else if (i >= n) i -= n;
     if ((unsigned)i >= (unsigned)n) i = ((i % n) + n) % n;
     return i;
-}
-
-// Exact bilinear fetch, LINEAR filter with REPEAT addressing
-// (src/RaytracingDescriptors.hpp:63, 70).
-template <int NC, class Tex>
-__device__ __forceinline__ void bilinear(const Tex& tex, uint32_t w, uint32_t h, float u, float v, float* out) {
-    float x = u * (float)w - 0.5f;
-    float y = v * (float)h - 0.5f;
-    float fx0 = floorf(x), fy0 = floorf(y);
-    float ax = x - fx0, ay = y - fy0;
-    int i0 = (int)fx0, j0 = (int)fy0;
-    int iw = (int)w, ih = (int)h;
-    int i1 = i0 + 1, j1 = j0 + 1;
-    i0 = wrap_repeat(i0, iw);
-    i1 = wrap_repeat(i1, iw);
-    j0 = wrap_repeat(j0, ih);
-    j1 = wrap_repeat(j1, ih);
-    float t00[NC], t10[NC], t01[NC], t11[NC];
-    tex.fetch((size_t)j0 * w + i0, t00);
-    tex.fetch((size_t)j0 * w + i1, t10);
-    tex.fetch((size_t)j1 * w + i0, t01);
-    tex.fetch((size_t)j1 * w + i1, t11);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        float top = t00[c] * (1.0f - ax) + t10[c] * ax;
-        float bot = t01[c] * (1.0f - ax) + t11[c] * ax;
-        out[c] = top * (1.0f - ay) + bot * ay;
-    }
 }
 
 }  // namespace ddgi

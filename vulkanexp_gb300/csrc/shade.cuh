@@ -80,10 +80,6 @@ struct AtlasView {
     DT depth;
 };
 
-__device__ __forceinline__ float3 grid_probe_pos(const DeviceGrid& g, int x, int y, int z) {
-    return f3((float)x * g.cell[0] + g.mn[0], (float)y * g.cell[1] + g.mn[1], (float)z * g.cell[2] + g.mn[2]);
-}
-
 // The lookup's arithmetic is written with explicit fmaf / __fmul_rn where a
 // product meets a sum, so that every kernel it is inlined into (single and
 // batched, FP32 and FP16 atlas) rounds alike.
@@ -118,11 +114,13 @@ __device__ __forceinline__ void sqrt_approx3(const float (&v)[3], float (&r)[3])
     }
 }
 
-// sphere_to_oct_uv (common.cuh) with one reciprocal for its quotients.  Each
-// quotient is brought to the correctly rounded one by its remainder (Markstein
-// 1990: q + (a - q b) / b with the reciprocal refined by a Newton step), so
-// the mapping has the bits of a division: next to a probe of strong contrast
-// one unit in the last place of uv shows in the result's sixth digit.
+// Octahedral coordinates of a direction of length one (irradiance.glsl:119-138)
+// with one reciprocal for its quotients.  Each quotient is brought to the
+// correctly rounded one by its remainder (Markstein 1990: q + (a - q b) / b
+// with the reciprocal refined by a Newton step), so the mapping has the bits
+// of a division (below 2^-102 a quotient can differ, which the added half
+// hides): next to a probe of strong contrast one unit in the last place of uv
+// shows in the result's sixth digit.
 __device__ __forceinline__ float2 oct_uv(float3 d) {
     const float sum = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
     float r = __fdividef(1.0f, sum);
@@ -144,8 +142,9 @@ __device__ __forceinline__ float2 oct_uv(float3 d) {
 // the texel position that times the atlas width, side x tiles, less half a
 // texel.  Here the quotient by `tiles` and its product are left out (exact
 // inverses of each other on grids of powers of two, one rounding less on the
-// others); the sum of tile and uv is rounded as the reference's, so the
-// fraction has the reference's bits.  A lookup stays at least half a texel
+// others); the sum of tile and uv is rounded as the reference's, so for sides
+// that are powers of two the fraction has the reference's bits (for others
+// 1 / side is rounded before the sum).  A lookup stays at least half a texel
 // inside its tile; the clamps keep a NaN's in the atlas too.
 struct Tap {
     uint32_t row0, row1;  // first texel in the upper and in the lower row
