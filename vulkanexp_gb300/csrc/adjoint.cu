@@ -161,9 +161,11 @@ constexpr int kLookupWords = 32;  // weights of two lookups' eight probes, per t
 // geometry and the depth atlas (constants here); d sqrt(c)/dc at c = 0 is
 // taken as 0 (such texels receive only zero radiance whatever the parameters).
 //
-// The first pass over the eight probes is the forward's and keeps the weights
-// (`w`: this thread's column of kLookupWords in shared memory); the second
-// fetches the colours again and scatters.  Bound by the L2's reductions, 64 a
+// The first pass over the eight probes has the forward's directions and weights
+// bit for bit (its colours differ in rounding: their roots are divided by, and
+// correctly rounded) and keeps the weights (`w`: this thread's column of
+// kLookupWords in shared memory); the second fetches the colours again and
+// scatters.  Bound by the L2's reductions, 64 a
 // hit: of four floats each, where single floats took 192.  524 K rays of a
 // room: 580 us with both passes over everything, a lookup at a time, and
 // single-float reductions; 247 us now.
@@ -179,9 +181,7 @@ __device__ __forceinline__ void sample_probes_vjp2(float3 position, const float3
     float W[2], Wf[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-        biased[q] = f3(fmaf(normal[q].x + toCamera.x, g.bias, position.x),
-                       fmaf(normal[q].y + toCamera.y, g.bias, position.y),
-                       fmaf(normal[q].z + toCamera.z, g.bias, position.z));
+        biased[q] = biased_position(position, normal[q], toCamera, g);
         nuv[q] = oct_uv(normal[q]);
         S[q] = Sf[q] = f3(0, 0, 0);
         W[q] = Wf[q] = 0.0f;
@@ -334,8 +334,7 @@ __global__ void __launch_bounds__(kAdjointThreads) k_ray_adjoint(DeviceScene sc,
                 float3 diffuse = s.albedo * (1.0f - 0.04f) * (1.0f - s.metal);
                 float3 g_base = shadowed ? gxi : gxi * fade;
                 float3 g_pbr = shadowed ? f3(0, 0, 0) : gxi * fade;
-                float3 reflectDir = dir - s.normal * (2.0f * dot3(s.normal, dir));
-                const float3 lookups[2] = {reflectDir, s.normal}, gout[2] = {g_base * spec, g_base * diffuse};
+                const float3 lookups[2] = {reflected(dir, s.normal), s.normal}, gout[2] = {g_base * spec, g_base * diffuse};
                 float3 value[2];  // reflection, indirect
                 sample_probes_vjp2(s.position, lookups, -dir, g, states, at, gout, gatlas, &s_weights[0][threadIdx.x],
                                    value);
