@@ -24,8 +24,9 @@ namespace ddgi {
 namespace {
 
 // Bound by instruction issue and, below half the HBM rate, by the latency of
-// the taps: six blocks of 128 per SM (80 registers) 82 us at 1920x1080, eight
-// 84 us, blocks of 256 without a bound 90 us.
+// the taps.  1920x1080 over a 16-bit atlas / 643x361 over an FP32 one (us): six
+// blocks of 128 per SM (72 and 80 registers) 87 / 37, eight 86 / 43, blocks of 256
+// without a bound 87 / 37.
 template <class AV>
 __global__ void __launch_bounds__(128, 6) k_final_gather(GatherArgs a, AV at) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

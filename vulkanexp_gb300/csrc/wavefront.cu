@@ -593,16 +593,23 @@ uint32_t persistent_blocks(const void* kernel, size_t smem, uint32_t cap_per_sm 
 }
 
 // Lanes per hit of the front-hit shading for at most `total` hits, from the
-// threads resident at a time (`slots`, 97,280 on 152 SMs).  Rooms of 128 rays a
-// probe, all probes, 1 / 2 / 4 lanes (us):
+// threads resident at a time (`slots`, 97,280 on 152 SMs).  The kernel by itself
+// in rooms of 128 rays a probe, all probes, 1 / 2 / 4 lanes (us):
 //   records      32,768         65,536         98,304         196,608
-//   FP32 atlas   21 / 13 / 13   25 / 17 / 23   27 / 30 / 33   59 / 46 / 54
-//   FP16 atlas   18 / 13 / 12   19 / 15 / 20   20 / 25 / 28   38 / 39 / 46
+//   FP32 atlas   21 / 13 / 13   25 / 17 / 23   28 / 31 / 34   60 / 46 / 62
+//   FP16 atlas   18 / 13 / 12   19 / 16 / 21   21 / 26 / 28   43 / 41 / 54
 // Four lanes win while they fit with the hits' usual share of the records, two
-// while the launch fits in a round and a half.  Beyond that the two-lane form
-// still wins over an FP32 atlas, where one lane's two lookups spill registers
-// (1,048,576 records: 208 / 196 us), until the work done twice costs more
-// (4,194,304: a 6.47 ms update is 0.2 % slower).
+// while the launch fits in a round and a half; beyond that one lane over an FP16
+// atlas.  Over an FP32 atlas, where one lane's two lookups spill registers, two
+// lanes go on.  Whole updates, two lanes against one (300 boxes in a room; a
+// terrain of 1,025 instances):
+//   records   98,304  131,072  196,608  262,144  524,288  1.05 M  2.1 M   4.2 M
+//   room      +2.1 %  0        -5.7 %   -0.7 %   -1.5 %   -2.4 %  -2.0 %  -1.5 %
+//   terrain   -1.5 %  +0.1 %   +0.4 %   -2.8 %   -1.3 %   -0.4 %  -0.4 %  0
+// They lose where one lane's threads fit in a round and two lanes' just do not,
+// which depends on the hits' share of the records, so no line avoids it.  The
+// largest launches are left to one lane: a terrain of 4,097 instances at 4.2 M
+// records 6,333 against 6,389 us, its scheduled frame of 3.1 M 1,540 against 1,560.
 uint32_t shade_lanes(uint32_t total, bool fp16_atlas) {
     const uint32_t slots = kShadeBlocksPerSm * 128u * sm_count();
     if (total <= slots / 3u) return 4u;
