@@ -11,11 +11,10 @@ using namespace ddgi;
 
 namespace {
 
-__device__ uint32_t mixed(uint32_t x) {  // a 32-bit finaliser (Stafford's variants of MurmurHash3's)
-    x ^= x >> 16;
-    x *= 0x7feb352du;
-    x ^= x >> 15;
-    x *= 0x846ca68bu;
+__device__ uint32_t mixed(uint32_t x) {  // spreads a counter: products with odd numbers, folded
+    x = (x + 1u) * 0x9E3779B9u;
+    x = (x ^ (x >> 15)) * 0x2545F491u;
+    x = (x ^ (x >> 13)) * 0x9E3779B9u;
     return x ^ (x >> 16);
 }
 
